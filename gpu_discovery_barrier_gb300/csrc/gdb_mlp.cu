@@ -1,15 +1,15 @@
 // Schedule selector: loading the network, and its training on the GPU.
 //
-// Training is full-batch Adam over a masked squared loss.  One step is
-// three kernels:
-//   k_mlp_fwd_bwd  one thread per sample: forward pass, output error and the
-//                  back-propagated errors of both hidden layers, stored
-//                  feature-major (act[f * n + s]);
-//   k_mlp_wgrad    one warp per gradient entry: the sum over samples of
-//                  (input activation x output error), accumulated in FP64
-//                  in a fixed lane-stride order and a fixed shuffle tree,
-//                  so gradients are bit-identical from run to run;
-//   k_mlp_adam     one thread per parameter.
+// Training is full-batch Adam over a masked squared loss.  One step is two
+// kernels:
+//   k_mlp_grad  a CTA takes tiles of 128 samples: forward and backward pass
+//               into shared memory, then the tile's share of every gradient
+//               entry from there (register tiles of 4 x 4 entries), kept in
+//               registers from tile to tile as a pair of floats;
+//   k_mlp_step  one warp per gradient entry: the CTAs' sums in a fixed order
+//               in FP64, then the Adam update of that parameter.
+// Tiles, lanes and sums have a fixed order, so gradients are bit-identical
+// from run to run.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -22,9 +22,6 @@ using namespace gdb;
 
 namespace {
 
-// Per-sample activation rows: xn 12, h1 32, h2 32, dh1 32, dh2 32, dy 6, loss 1.
-constexpr int kAXn = 0, kAH1 = kAXn + kFeat, kAH2 = kAH1 + kH1, kADh1 = kAH2 + kH2,
-              kADh2 = kADh1 + kH1, kADy = kADh2 + kH2, kALoss = kADy + kOut, kActRows = kALoss + 1;
 // Gradient entries: W1, b1, W2, b2, W3, b3 (the blob minus shift/scale), then the loss.
 constexpr int kGradEntries = kParams - kPW1;
 
@@ -58,108 +55,357 @@ __global__ void k_mlp_forward(const float* __restrict__ p, const float* __restri
   for (int j = 0; j < kOut; ++j) Y[(size_t)s * kOut + j] = y[j];
 }
 
-__global__ void k_mlp_fwd_bwd(const float* __restrict__ p, const float* __restrict__ X,
-                              const float* __restrict__ T, const float* __restrict__ M, uint32_t n,
-                              float inv_m, float* __restrict__ act) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  float x[kFeat], xn[kFeat], h1[kH1], h2[kH2], y[kOut], dy[kOut];
-  for (int i = 0; i < kFeat; ++i) x[i] = X[(size_t)s * kFeat + i];
-  mlp_thread(p, x, xn, h1, h2, y);
-  float loss = 0.f;
-  for (int j = 0; j < kOut; ++j) {
-    const float m = M[(size_t)s * kOut + j];
-    const float e = y[j] - T[(size_t)s * kOut + j];
-    dy[j] = m != 0.f ? 2.f * m * e * inv_m : 0.f;
-    if (m != 0.f) loss = __fmaf_rn(m * e, e * inv_m, loss);
-  }
-  auto put = [&](int row, float v) { act[(size_t)row * n + s] = v; };
-  for (int i = 0; i < kFeat; ++i) put(kAXn + i, xn[i]);
-  for (int j = 0; j < kH1; ++j) put(kAH1 + j, h1[j]);
-  for (int j = 0; j < kH2; ++j) put(kAH2 + j, h2[j]);
-  for (int j = 0; j < kOut; ++j) put(kADy + j, dy[j]);
-  put(kALoss, loss);
-  // dh2 = W3 . dy masked by ReLU; dh1 = W2 . dh2 masked by ReLU
-  float dh2[kH2];
-  for (int k = 0; k < kH2; ++k) {
-    float a = 0.f;
-    for (int j = 0; j < kOut; ++j) a = __fmaf_rn(p[kPW3 + k * kOut + j], dy[j], a);
-    dh2[k] = h2[k] > 0.f ? a : 0.f;
-    put(kADh2 + k, dh2[k]);
-  }
-  for (int k = 0; k < kH1; ++k) {
-    float a = 0.f;
-    for (int j = 0; j < kH2; ++j) a = __fmaf_rn(p[kPW2 + k * kH2 + j], dh2[j], a);
-    put(kADh1 + k, h1[k] > 0.f ? a : 0.f);
+// Sum of the mask, in FP64 with a fixed order: one partial per CTA here,
+// the CTAs' partials in order in mask_inverse.
+constexpr int kMaskCtas = 64;
+__global__ void k_mask_sum(const float* __restrict__ m, size_t count, double* __restrict__ part) {
+  __shared__ double warp[8];
+  double a = 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
+    a += (double)m[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0) warp[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) a += warp[w];
+    part[blockIdx.x] = a;
   }
 }
 
-// Gradient entry e (0-based over W1, b1, W2, b2, W3, b3) as a pair of
-// activation rows (a row < 0 means the constant 1 of a bias).
-__device__ __forceinline__ void grad_rows(int e, int& ra, int& rd) {
-  if (e < kFeat * kH1) {
-    ra = kAXn + e / kH1;
-    rd = kADh1 + e % kH1;
-    return;
-  }
-  e -= kFeat * kH1;
-  if (e < kH1) {
-    ra = -1;
-    rd = kADh1 + e;
-    return;
-  }
-  e -= kH1;
-  if (e < kH1 * kH2) {
-    ra = kAH1 + e / kH2;
-    rd = kADh2 + e % kH2;
-    return;
-  }
-  e -= kH1 * kH2;
-  if (e < kH2) {
-    ra = -1;
-    rd = kADh2 + e;
-    return;
-  }
-  e -= kH2;
-  if (e < kH2 * kOut) {
-    ra = kAH2 + e / kOut;
-    rd = kADy + e % kOut;
-    return;
-  }
-  e -= kH2 * kOut;
-  ra = -1;
-  rd = kADy + e;
+// Rows of a tile's activations in shared memory (kTile samples each): the
+// normalised features, both hidden layers, their back-propagated errors,
+// the output errors and the samples' losses.
+constexpr int kTile = 128;
+constexpr int kPitch = kTile + 4;  // rows 16-byte aligned, eight neighbouring rows on distinct banks
+constexpr int kRXn = 0, kRH1 = kRXn + kFeat, kRH2 = kRH1 + kH1, kRDh1 = kRH2 + kH2, kRDh2 = kRDh1 + kH1,
+              kRDy = kRDh2 + kH2, kRLoss = kRDy + kOut, kRows = kRLoss + 1;
+constexpr int kMlpThreads = 256;
+constexpr int kMlpSmem = (kRows * kPitch + ((kRows + 3) & ~3) + ((kParams + 3) & ~3)) * 4;
+static_assert(kPW1 % 4 == 0 && kPW2 % 4 == 0, "weight rows are read as float4");
+
+// Exact-to-2^-48 accumulation of one more term into the pair (hi, lo).
+__device__ __forceinline__ void pair_add(float& hi, float& lo, float x) {
+  const float t = __fadd_rn(hi, x), z = __fsub_rn(t, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(x, z)));
+  hi = t;
 }
 
-__global__ void k_mlp_wgrad(const float* __restrict__ act, uint32_t n, float* __restrict__ grad,
-                            double* __restrict__ loss) {
+// Forward pass, errors and gradient sums of the CTA's tiles.  The gradient
+// is the contraction of activation rows with error rows over the samples.
+// It was one warp per entry with an FP64 FMA per (entry, sample) and both
+// rows re-read from L2: 135,000 samples took 1.9 ms a step, bound by the
+// FP64 pipe and the 1,694 x 2 row reads.  Here
+//  * the rows stay in shared memory: a thread holds 4 x 4 entries and reads
+//    eight 16-byte row pieces per four samples; tiles' rows interleave (t,
+//    t + 8, ...), so a warp's eight distinct rows fall on distinct banks;
+//  * FP64's place is taken by error-free extraction against a fixed grid
+//    (Rump, Ogita, Oishi, "Accurate floating-point summation", SIAM J. Sci.
+//    Comput. 31(1), 2008): with C = 1.5 x 2^k above the sum of the tile's
+//    |products| (from the rows' largest magnitudes), acc = fma(a, b, acc)
+//    rounds a product onto C's grid, acc' - acc is that part exactly, and
+//    fma(a, b, -part) the rest, which goes to a second float.  Four FP32
+//    operations per product, an error near 2^-35 of the largest product
+//    (below the 2^-24 of the float gradient).  Where the grid would
+//    overflow, the thread sums its tile in FP64 instead.
+// 135,000 samples: 1.9 -> 0.11 ms a step, k_mlp_step included.
+__global__ void __launch_bounds__(kMlpThreads, 2)
+    k_mlp_grad(const float* __restrict__ p, const float* __restrict__ X, const float* __restrict__ T,
+               const float* __restrict__ M, uint32_t n, const float* __restrict__ inv_mask,
+               double* __restrict__ part) {
+  extern __shared__ float4 mlp_smem[];
+  float* act = reinterpret_cast<float*>(mlp_smem);  // [kRows][kPitch]
+  float* top = act + kRows * kPitch;                // [kRows] largest magnitude of a row
+  float* sp = top + ((kRows + 3) & ~3);             // the parameters
+  const int tid = threadIdx.x;
+  const float inv_m = __ldg(inv_mask);
+  for (int i = tid; i < kParams; i += kMlpThreads) sp[i] = __ldg(&p[i]);
+
+  // phase 1 takes two samples and a quarter of each layer per thread
+  const int quarter = (tid >> 6) * 8, sa = tid & 63, sb = sa + 64;
+
+  // phase 2: 104 tiles of 4 x 4 entries, each over both halves of the
+  // samples, on threads 0-207; the column sums (biases, loss) on the rest
+  const bool tiled = tid < 208;
+  int half, a0, as, d0, ds, out0, outw, ocol, nd = 4;
+  if (tid < 128) {  // W2: h1 x dh2
+    const int t = tid & 63;
+    half = tid >> 6;
+    a0 = kRH1 + (t >> 3), as = 8, d0 = kRDh2 + (t & 7), ds = 8;
+    out0 = kPW2 + (t >> 3) * kH2 + (t & 7), outw = 8 * kH2, ocol = 8;
+  } else if (tid < 176) {  // W1: xn x dh1
+    const int t = (tid - 128) % 24;
+    half = (tid - 128) / 24;
+    a0 = kRXn + (t >> 3), as = 3, d0 = kRDh1 + (t & 7), ds = 8;
+    out0 = kPW1 + (t >> 3) * kH1 + (t & 7), outw = 3 * kH1, ocol = 8;
+  } else {  // W3: h2 x dy (three of the six columns; the last one is read twice)
+    const int t = (tid - 176) & 15;
+    half = ((tid - 176) >> 4) & 1;
+    a0 = kRH2 + (t >> 1), as = 8, d0 = kRDy + (t & 1), ds = 2;
+    out0 = kPW3 + (t >> 1) * kOut + (t & 1), outw = 8 * kOut, ocol = 2;
+    nd = 3;
+  }
+  // error row of column j: its offset from row d0
+  const int d3 = (nd - 1) * ds;
+  auto drow = [&](int j) { return j < 3 ? j * ds : d3; };
+  const int colr0 = tid - 208, colr1 = colr0 + 48;  // column sums: rows of dh1, dh2, dy, loss from kRDh1
+  constexpr int kCols = kRows - kRDh1;
+  float rhi[16], rlo[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) rhi[i] = rlo[i] = 0.f;
+
+  for (uint32_t tile = blockIdx.x; (size_t)tile * kTile < n; tile += gridDim.x) {
+    const size_t base = (size_t)tile * kTile;
+    const uint32_t have = n - base < (size_t)kTile ? (uint32_t)(n - base) : (uint32_t)kTile;
+    // targets and masks of thread tid < 128's sample, in flight early
+    float tt[kOut], mm[kOut];
+    if (tid < kTile) {
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        tt[j] = (uint32_t)tid < have ? __ldg(&T[(base + tid) * kOut + j]) : 0.f;
+        mm[j] = (uint32_t)tid < have ? __ldg(&M[(base + tid) * kOut + j]) : 0.f;
+      }
+    }
+    __syncthreads();  // the previous tile's rows (and the parameters) are done with (in place)
+    for (int i = tid; i < kTile * kFeat; i += kMlpThreads) {
+      const int s = i / kFeat, f = i - s * kFeat;
+      act[(kRXn + f) * kPitch + s] =
+          (uint32_t)s < have ? __fmul_rn(__fsub_rn(__ldg(&X[base * kFeat + i]), sp[kPShift + f]), sp[kPScale + f])
+                             : 0.f;
+    }
+    __syncthreads();
+    // one layer: outputs quarter .. quarter + 7 of both samples
+    auto layer = [&](int rin, int nin, const float* w, const float* bias, int rout) {
+      float ha[8], hb[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ha[j] = hb[j] = bias[quarter + j];
+#pragma unroll 4
+      for (int i = 0; i < nin; ++i) {
+        const float xa = act[(rin + i) * kPitch + sa], xb = act[(rin + i) * kPitch + sb];
+        const float4 w0 = *reinterpret_cast<const float4*>(&w[i * 32 + quarter]);
+        const float4 w1 = *reinterpret_cast<const float4*>(&w[i * 32 + quarter + 4]);
+        const float wj[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          ha[j] = __fmaf_rn(xa, wj[j], ha[j]);
+          hb[j] = __fmaf_rn(xb, wj[j], hb[j]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        act[(rout + quarter + j) * kPitch + sa] = fmaxf(ha[j], 0.f);
+        act[(rout + quarter + j) * kPitch + sb] = fmaxf(hb[j], 0.f);
+      }
+      __syncthreads();
+    };
+    layer(kRXn, kFeat, sp + kPW1, sp + kPB1, kRH1);
+    layer(kRH1, kH1, sp + kPW2, sp + kPB2, kRH2);
+    if (tid < kTile) {
+      float y[kOut];
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) y[j] = sp[kPB3 + j];
+#pragma unroll 4
+      for (int k = 0; k < kH2; ++k) {
+        const float h = act[(kRH2 + k) * kPitch + tid];
+#pragma unroll
+        for (int j = 0; j < kOut; ++j) y[j] = __fmaf_rn(h, sp[kPW3 + k * kOut + j], y[j]);
+      }
+      float loss = 0.f;
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        const float e = y[j] - tt[j];
+        act[(kRDy + j) * kPitch + tid] = mm[j] != 0.f ? 2.f * mm[j] * e * inv_m : 0.f;
+        if (mm[j] != 0.f) loss = __fmaf_rn(mm[j] * e, e * inv_m, loss);
+      }
+      act[kRLoss * kPitch + tid] = loss;
+    }
+    __syncthreads();
+    // dh2 = W3 . dy and dh1 = W2 . dh2, each masked by its ReLU
+    {
+      float da[kOut], db[kOut];
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        da[j] = act[(kRDy + j) * kPitch + sa];
+        db[j] = act[(kRDy + j) * kPitch + sb];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = quarter + i;
+        float a = 0.f, b = 0.f;
+#pragma unroll
+        for (int j = 0; j < kOut; ++j) {
+          const float w = sp[kPW3 + k * kOut + j];
+          a = __fmaf_rn(w, da[j], a);
+          b = __fmaf_rn(w, db[j], b);
+        }
+        act[(kRDh2 + k) * kPitch + sa] = act[(kRH2 + k) * kPitch + sa] > 0.f ? a : 0.f;
+        act[(kRDh2 + k) * kPitch + sb] = act[(kRH2 + k) * kPitch + sb] > 0.f ? b : 0.f;
+      }
+    }
+    __syncthreads();
+    {
+      float a[8], b[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = b[i] = 0.f;
+#pragma unroll 2
+      for (int j = 0; j < kH2; j += 4) {
+        float da[4], db[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          da[q] = act[(kRDh2 + j + q) * kPitch + sa];
+          db[q] = act[(kRDh2 + j + q) * kPitch + sb];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(&sp[kPW2 + (quarter + i) * kH2 + j]);
+          const float wq[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            a[i] = __fmaf_rn(wq[q], da[q], a[i]);
+            b[i] = __fmaf_rn(wq[q], db[q], b[i]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = quarter + i;
+        act[(kRDh1 + k) * kPitch + sa] = act[(kRH1 + k) * kPitch + sa] > 0.f ? a[i] : 0.f;
+        act[(kRDh1 + k) * kPitch + sb] = act[(kRH1 + k) * kPitch + sb] > 0.f ? b[i] : 0.f;
+      }
+    }
+    __syncthreads();
+    for (int r = tid >> 5; r < kRows; r += kMlpThreads / 32) {
+      const float4 v = *reinterpret_cast<const float4*>(&act[r * kPitch + 4 * (tid & 31)]);
+      // magnitudes order as their bits do, NaN above infinity
+      const uint32_t m = max(max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.y))),
+                             max(__float_as_uint(fabsf(v.z)), __float_as_uint(fabsf(v.w))));
+      const uint32_t w = __reduce_max_sync(0xffffffffu, m);
+      if ((tid & 31) == 0) top[r] = __uint_as_float(w);
+    }
+    __syncthreads();
+    if (tiled) {
+      // C = 1.5 x 2^k with 2^k above twice the largest possible |sum| of
+      // the 64 products, so acc keeps C's exponent throughout
+      auto grid_of = [&](int i, int j) {
+        const float b = top[a0 + i * as] * top[d0 + drow(j)] * 160.f;
+        return 1.5f * __uint_as_float((__float_as_uint(b) & 0x7f800000u) + 0x00800000u);
+      };
+      bool fits = true;
+      float acc[16], lo[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          fits = fits && top[a0 + i * as] * top[d0 + drow(j)] < 1e34f;
+          acc[4 * i + j] = grid_of(i, j);
+          lo[4 * i + j] = 0.f;
+        }
+      const float* A = act + a0 * kPitch + 64 * half;
+      const float* D = act + d0 * kPitch + 64 * half;
+      if (fits) {
+#pragma unroll 1
+        for (int s = 0; s < 64; s += 4) {
+          float av[4][4], dv[4][4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(A + i * as * kPitch + s);
+            const float4 y = *reinterpret_cast<const float4*>(D + drow(i) * kPitch + s);
+            av[i][0] = x.x, av[i][1] = x.y, av[i][2] = x.z, av[i][3] = x.w;
+            dv[i][0] = y.x, dv[i][1] = y.y, dv[i][2] = y.z, dv[i][3] = y.w;
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int e = 4 * i + j;
+                const float t = __fmaf_rn(av[i][q], dv[j][q], acc[e]);
+                const float on = __fsub_rn(t, acc[e]);
+                lo[e] = __fadd_rn(lo[e], __fmaf_rn(av[i][q], dv[j][q], -on));
+                acc[e] = t;
+              }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int e = 4 * i + j;
+            pair_add(rhi[e], rlo[e], __fsub_rn(acc[e], grid_of(i, j)));
+            pair_add(rhi[e], rlo[e], lo[e]);
+          }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            double sum = 0.0;
+#pragma unroll 1
+            for (int s = 0; s < 64; ++s) sum += (double)A[i * as * kPitch + s] * (double)D[drow(j) * kPitch + s];
+            const float f = (float)sum;
+            pair_add(rhi[4 * i + j], rlo[4 * i + j], f);
+            pair_add(rhi[4 * i + j], rlo[4 * i + j], (float)(sum - (double)f));
+          }
+      }
+    } else {
+      const float* c0 = act + (kRDh1 + colr0) * kPitch;
+      const float* c1 = act + (kRDh1 + (colr1 < kCols ? colr1 : colr0)) * kPitch;
+#pragma unroll 4
+      for (int s = 0; s < kTile; ++s) {
+        pair_add(rhi[0], rlo[0], c0[s]);
+        pair_add(rhi[1], rlo[1], c1[s]);
+      }
+    }
+  }
+  // part[entry][slot]: two slots per CTA, one per half of the samples
+  const size_t slots = 2 * (size_t)gridDim.x;
+  if (tiled) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < nd)
+          part[(size_t)(out0 - kPW1 + i * outw + j * ocol) * slots + 2 * blockIdx.x + half] =
+              (double)rhi[4 * i + j] + (double)rlo[4 * i + j];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = k ? colr1 : colr0;
+      if (c >= kCols) break;
+      // dh1, dh2 and dy columns are the biases; the loss is the last entry
+      const int e = c < kH1 ? kPB1 + c : c < kH1 + kH2 ? kPB2 + c - kH1
+                  : c < kH1 + kH2 + kOut ? kPB3 + c - kH1 - kH2 : kParams;
+      double* o = part + (size_t)(e - kPW1) * slots + 2 * blockIdx.x;
+      o[0] = (double)rhi[k] + (double)rlo[k];
+      o[1] = 0.0;
+    }
+  }
+}
+
+// The CTAs' sums of one entry per warp, in a fixed order, then (m1 != null)
+// the Adam update of its parameter.
+__global__ void k_mlp_step(const double* __restrict__ part, int slots, float* __restrict__ grad,
+                           double* __restrict__ loss, float* __restrict__ p, float* __restrict__ m1,
+                           float* __restrict__ m2, float lr_t, float wd) {
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (e > kGradEntries) return;
   double acc = 0.0;
-  if (e == kGradEntries) {
-    for (uint32_t s = lane; s < n; s += 32) acc += (double)act[(size_t)kALoss * n + s];
-  } else {
-    int ra, rd;
-    grad_rows(e, ra, rd);
-    const float* A = ra >= 0 ? act + (size_t)ra * n : nullptr;
-    const float* D = act + (size_t)rd * n;
-    for (uint32_t s = lane; s < n; s += 32) acc += (A ? (double)A[s] : 1.0) * (double)D[s];
-  }
+  for (int s = lane; s < slots; s += 32) acc += part[(size_t)e * slots + s];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) {
-    if (e == kGradEntries) *loss = acc;
-    else grad[kPW1 + e] = (float)acc;
+  if (lane != 0) return;
+  if (e == kGradEntries) {
+    *loss = acc;
+    return;
   }
-}
-
-__global__ void k_mlp_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
-                           float* __restrict__ m2, float lr_t, float wd) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < kPW1 || i >= kParams) return;
-  const bool weight = (i >= kPW1 && i < kPB1) || (i >= kPW2 && i < kPB2) || (i >= kPW3 && i < kPB3);
-  float gi = g[i];
+  const int i = kPW1 + e;
+  if (!m1) {
+    grad[i] = (float)acc;
+    return;
+  }
+  const bool weight = i < kPB1 || (i >= kPW2 && i < kPB2) || (i >= kPW3 && i < kPB3);
+  float gi = (float)acc;
   if (weight) gi += wd * p[i];
   m1[i] = 0.9f * m1[i] + 0.1f * gi;
   m2[i] = 0.999f * m2[i] + 0.001f * gi * gi;
@@ -168,34 +414,49 @@ __global__ void k_mlp_adam(float* __restrict__ p, const float* __restrict__ g, f
 
 // Device buffers of one training / gradient call.
 struct MlpBufs {
-  float *p = nullptr, *x = nullptr, *t = nullptr, *m = nullptr, *act = nullptr, *g = nullptr,
-        *m1 = nullptr, *m2 = nullptr;
-  double* loss = nullptr;
+  float *p = nullptr, *x = nullptr, *t = nullptr, *m = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr,
+        *inv_mask = nullptr;
+  double *loss = nullptr, *part = nullptr;
   char* base = nullptr;
+  int ctas = 0;
 };
+
+// 1 / sum of the mask (0 for an empty one).
+__global__ void k_mask_inverse(const double* __restrict__ part, float* __restrict__ inv) {
+  double s = 0.0;
+  for (int i = 0; i < kMaskCtas; ++i) s += part[i];
+  *inv = s > 0 ? (float)(1.0 / s) : 0.f;
+}
 
 int mlp_upload(gdb_ctx* c, MlpBufs& b, const float* params, const float* x, const float* t,
                const float* m, uint32_t n, bool adam) {
+  // two CTAs per SM hold the tiles; fewer tiles take a CTA each
+  b.ctas = (int)std::min<uint64_t>(2ull * c->sm_count, ((uint64_t)n + kTile - 1) / kTile);
+  GDB_CUDA(c, cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlpSmem));
   Bump bp;
   const size_t o_p = bp.take(kParams * 4), o_x = bp.take((size_t)n * kFeat * 4),
                o_t = bp.take((size_t)n * kOut * 4), o_m = bp.take((size_t)n * kOut * 4),
-               o_a = bp.take((size_t)n * kActRows * 4), o_g = bp.take(kParams * 4),
-               o_m1 = bp.take(adam ? kParams * 4 : 0), o_m2 = bp.take(adam ? kParams * 4 : 0),
-               o_l = bp.take(8);
+               o_g = bp.take(kParams * 4), o_m1 = bp.take(adam ? kParams * 4 : 0),
+               o_m2 = bp.take(adam ? kParams * 4 : 0), o_l = bp.take(8), o_i = bp.take(4),
+               o_s = bp.take((size_t)std::max((kGradEntries + 1) * 2 * b.ctas, kMaskCtas) * 8);
   GDB_CUDA(c, cudaMallocAsync((void**)&b.base, bp.off, c->stream));
   b.p = (float*)(b.base + o_p);
   b.x = (float*)(b.base + o_x);
   b.t = (float*)(b.base + o_t);
   b.m = (float*)(b.base + o_m);
-  b.act = (float*)(b.base + o_a);
   b.g = (float*)(b.base + o_g);
-  b.m1 = (float*)(b.base + o_m1);
-  b.m2 = (float*)(b.base + o_m2);
+  b.m1 = adam ? (float*)(b.base + o_m1) : nullptr;
+  b.m2 = adam ? (float*)(b.base + o_m2) : nullptr;
   b.loss = (double*)(b.base + o_l);
+  b.inv_mask = (float*)(b.base + o_i);
+  b.part = (double*)(b.base + o_s);
   GDB_CUDA(c, cudaMemcpyAsync(b.p, params, kParams * 4, cudaMemcpyHostToDevice, c->stream));
+  GDB_CUDA(c, cudaMemcpyAsync(b.m, m, (size_t)n * kOut * 4, cudaMemcpyHostToDevice, c->stream));
+  k_mask_sum<<<kMaskCtas, 256, 0, c->stream>>>(b.m, (size_t)n * kOut, b.part);
+  k_mask_inverse<<<1, 1, 0, c->stream>>>(b.part, b.inv_mask);
+  GDB_CUDA(c, cudaGetLastError());
   GDB_CUDA(c, cudaMemcpyAsync(b.x, x, (size_t)n * kFeat * 4, cudaMemcpyHostToDevice, c->stream));
   GDB_CUDA(c, cudaMemcpyAsync(b.t, t, (size_t)n * kOut * 4, cudaMemcpyHostToDevice, c->stream));
-  GDB_CUDA(c, cudaMemcpyAsync(b.m, m, (size_t)n * kOut * 4, cudaMemcpyHostToDevice, c->stream));
   GDB_CUDA(c, cudaMemsetAsync(b.g, 0, kParams * 4, c->stream));
   if (adam) {
     GDB_CUDA(c, cudaMemsetAsync(b.m1, 0, kParams * 4, c->stream));
@@ -204,17 +465,13 @@ int mlp_upload(gdb_ctx* c, MlpBufs& b, const float* params, const float* x, cons
   return GDB_OK;
 }
 
-int mlp_step(gdb_ctx* c, MlpBufs& b, uint32_t n, float inv_m) {
-  k_mlp_fwd_bwd<<<(n + 127) / 128, 128, 0, c->stream>>>(b.p, b.x, b.t, b.m, n, inv_m, b.act);
-  k_mlp_wgrad<<<(kGradEntries + 1 + 7) / 8, 256, 0, c->stream>>>(b.act, n, b.g, b.loss);
+// Gradient and loss, then the Adam update where b has its moments.
+int mlp_step(gdb_ctx* c, MlpBufs& b, uint32_t n, float lr_t, float wd) {
+  k_mlp_grad<<<b.ctas, kMlpThreads, kMlpSmem, c->stream>>>(b.p, b.x, b.t, b.m, n, b.inv_mask, b.part);
+  k_mlp_step<<<(kGradEntries + 1 + 7) / 8, 256, 0, c->stream>>>(b.part, 2 * b.ctas, b.g, b.loss, b.p, b.m1,
+                                                                b.m2, lr_t, wd);
   GDB_CUDA(c, cudaGetLastError());
   return GDB_OK;
-}
-
-float mask_inverse(const float* m, uint32_t n) {
-  double s = 0;
-  for (size_t i = 0; i < (size_t)n * kOut; ++i) s += m[i];
-  return s > 0 ? (float)(1.0 / s) : 0.f;
 }
 
 }  // namespace
@@ -261,7 +518,7 @@ int gdb_mlp_loss_grad(gdb_ctx* c, const float* params, const float* x, const flo
   if (!c || !params || !x || !t || !m || !grad || n == 0) return GDB_ERR_INVALID;
   MlpBufs b;
   int rc = mlp_upload(c, b, params, x, t, m, n, false);
-  if (rc == GDB_OK) rc = mlp_step(c, b, n, mask_inverse(m, n));
+  if (rc == GDB_OK) rc = mlp_step(c, b, n, 0.f, 0.f);
   cudaError_t e = cudaSuccess;
   if (rc == GDB_OK) {
     e = cudaMemcpyAsync(grad, b.g, kParams * 4, cudaMemcpyDeviceToHost, c->stream);
@@ -278,17 +535,11 @@ int gdb_mlp_train(gdb_ctx* c, float* params, const float* x, const float* t, con
   if (!c || !params || !x || !t || !m || n == 0 || !(lr > 0.f)) return GDB_ERR_INVALID;
   MlpBufs b;
   int rc = mlp_upload(c, b, params, x, t, m, n, true);
-  const float inv_m = mask_inverse(m, n);
   double b1t = 1.0, b2t = 1.0;
   for (uint32_t k = 0; rc == GDB_OK && k < epochs; ++k) {
-    rc = mlp_step(c, b, n, inv_m);
-    if (rc) break;
     b1t *= 0.9;
     b2t *= 0.999;
-    const float lr_t = (float)(lr * std::sqrt(1.0 - b2t) / (1.0 - b1t));
-    k_mlp_adam<<<(kParams + 255) / 256, 256, 0, c->stream>>>(b.p, b.g, b.m1, b.m2, lr_t, wd);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) rc = set_cuda_error(c, e, "mlp adam");
+    rc = mlp_step(c, b, n, (float)(lr * std::sqrt(1.0 - b2t) / (1.0 - b1t)), wd);
   }
   cudaError_t e = cudaSuccess;
   if (rc == GDB_OK) {
