@@ -37,6 +37,7 @@
 //    change flag, so an iteration costs one barrier instead of three.
 #include <algorithm>
 
+#include "gdb_drain.cuh"
 #include "gdb_internal.h"
 #include "gdb_relaunch.cuh"
 #include "gdb_selector.cuh"
@@ -90,6 +91,8 @@ struct SsspWs {
   gdb_level_trace* trace;      // one record per settle superstep (nullable)
   uint32_t trace_cap;
   uint32_t maxdeg;
+  uint32_t share;     // vertices per CTA up to which a superstep without the split may be narrow
+  uint32_t patience;  // such supersteps in a row before the first that is
 };
 
 enum { kSettleRule = 0, kSettleLearned = 1, kSettlePush = 2, kSettlePull = 3 };
@@ -183,6 +186,7 @@ __device__ __forceinline__ uint32_t dist_of(const SsspWs& ws, uint32_t v) {
 // (light, packed heavy, pile size, pile minimum), loaded once per CTA into
 // shared memory; every thread of the CTA calls it and reads the words
 // until the next call.
+template <bool MaySplit>
 __device__ __forceinline__ const unsigned long long* step_counts(const SsspWs& ws, int cur,
                                                                  uint32_t phase) {
   __shared__ unsigned long long s[7];
@@ -192,7 +196,7 @@ __device__ __forceinline__ const unsigned long long* step_counts(const SsspWs& w
     s[1] = __ldcg(&ws.hcount[cur]);
     s[2] = ws.delta ? ld_cg(&ws.farcount[phase % 3]) : 0u;
     s[3] = ws.delta ? ld_cg(&ws.farmin[phase % 3]) : 0u;
-    const bool split = ws.light < kInf;
+    const bool split = MaySplit && ws.light < kInf;
     s[4] = split ? ld_cg(ws.sqcount) : 0u;
     s[5] = split ? (uint32_t)__ldcg(ws.shcount) : 0u;
     s[6] = split ? __ldcg(ws.sarcs) : 0ull;
@@ -458,25 +462,85 @@ __device__ __forceinline__ void far_filter(const GraphView& G, const Warps& W, c
   if (lane == 0 && fmin != 0xFFFFFFFFu) atomicMin(&ws.farmin[(phase + 1) % 3], fmin);
 }
 
+// 4096^2 grid at width 16,016 with 448 / 640 / 768 / 1,024 slots: 34.2 / 26.1 /
+// 23.8 / 21.2 ms (a bucket's near entries outgrow the smaller ones).
+using SsspDrain = DrainMem<1024, 512>;
+
+// Narrow superstep of a run without the split (gdb_drain.cuh).  dry: the
+// bucket has run out and [lo, split) of the far pile follows (fn entries of
+// the pile of phase - 1; kept entries and far improvements go to the pile
+// of `phase`); otherwise the near queue's n vertices.  Spilled vertices
+// enter superstep L + 1's frontier once (stamp).
+__device__ __forceinline__ void sssp_narrow(const GraphView& G, const SsspWs& ws, SsspDrain& m, int id, int P,
+                                            uint32_t L, uint32_t lo, uint32_t split, uint32_t phase, bool dry,
+                                            uint32_t n, unsigned long long& arcs) {
+  const int lane = lane_id(), nxt = (L + 1) % 3;
+  const Frontier out{pick(ws.q, L + 1), pick(ws.hc, L + 1), &ws.qcount[nxt], &ws.hcount[nxt],
+                     ws.qcap, ws.hcap, ws.overflow};
+  const uint32_t pile = phase + 1;
+  uint32_t fmin = 0xFFFFFFFFu;
+  auto far = [&](bool want, uint32_t v) {
+    far_push(ws, phase, want && atomicExch(&ws.farmark[v], pile) != pile, v);
+  };
+  auto spill = [&](bool want, uint32_t v) {
+    frontier_push(G, out, want && atomicExch(&ws.stamp[v], L + 1) != L + 1, v);
+  };
+  auto label = [&](uint32_t v) { return dist_of<true>(ws, v); };
+  drain_reset(m);
+  if (dry) {
+    const uint32_t* from = pick(ws.far, phase - 1);
+    const uint32_t have = drain_items(n, P);
+    for (uint32_t base = threadIdx.x & ~31u; base < have; base += blockDim.x) {
+      const uint32_t i = drain_item(base + lane, id, P);
+      const bool act = base + lane < have && i < n;
+      const uint32_t v = act ? ld_cg(&from[i]) : 0u;
+      const uint32_t d = act ? label(v) : 0u;
+      const bool near = act && d >= lo && d < split, keep = act && d >= split;
+      bool over = false;
+      if (near) {
+        const uint32_t r0 = __ldg(&G.row[v]), r1 = __ldg(&G.row[v + 1]);
+        over = is_heavy(G, v) || !drain_add(m, 0, 0, v, d, r0, r1 - r0);
+      }
+      if (__any_sync(kFull, over)) spill(over, v);
+      if (keep) fmin = min(fmin, d);
+      far(keep, v);
+    }
+  } else {
+    drain_take(G, m, pick(ws.q, L), n, id, P, label, spill);
+  }
+  const uint32_t hops = drain_run(
+      G, m, split, fmin, arcs, [&](uint32_t arc) { return __ldg(&G.w[arc]); }, label,
+      [&](uint32_t v, uint32_t d) {
+        return (uint32_t)(atomicMin(&ws.key[v], (unsigned long long)d << 32) >> 32);
+      },
+      far, spill);
+  if (ws.delta) {
+    fmin = __reduce_min_sync(kFull, fmin);
+    if (lane == 0 && fmin != 0xFFFFFFFFu) atomicMin(&ws.farmin[phase % 3], fmin);
+  }
+  if (threadIdx.x == 0) atomicMax(&ws.cursor[L % 3], hops);
+}
+
 // G: the arcs near supersteps relax (all arcs, or the light half under
 // the split); GH: the heavy half the settle supersteps relax, GT the same
 // transposed (split only).
 // Hooked: the settle direction comes from settle_choose (learned and trace
 // schedules); a separate instantiation keeps the plain kernels' registers.
-template <bool Hooked, class Sync>
+// Narrow: a run without the split, whose small supersteps are narrow ones.
+template <bool Hooked, bool Narrow, class Sync>
 __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const GraphView& GH,
                                           const GraphView& GT, const SsspWs& ws, uint32_t src,
-                                          uint32_t* smin, SettleState* sst) {
+                                          uint32_t* smin, SettleState* sst, SsspDrain* drain) {
   const Warps W = warps_of(s.id(), s.P());
   const bool leader = s.id() == 0 && threadIdx.x == 0;
-  const bool split_arcs = ws.light < kInf;
+  const bool split_arcs = !Narrow && ws.light < kInf;
   if constexpr (Hooked) {
     if (threadIdx.x == 0) *sst = SettleState{0, 0, 0};  // read after the first barrier
   }
   for (uint32_t v = W.gthread; v < G.V; v += W.nthreads) {
     ws.key[v] = (unsigned long long)kInf << 32;
     if (ws.delta) ws.farmark[v] = 0;
-    if (split_arcs) ws.stamp[v] = 0;
+    if (Narrow || split_arcs) ws.stamp[v] = 0;
   }
   if (leader) {
     for (int i = 0; i < 3; ++i) {
@@ -524,9 +588,13 @@ __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const Gra
   uint32_t sdone = 0, hdone = 0;
   unsigned long long adone = 0;
   const uint32_t whi = split_arcs ? ws.light : kInf;
+  // supersteps reported: a narrow one counts the hops of its longest CTA
+  // (left in the superstep's cursor word, which it does not use otherwise)
+  uint32_t inner = 0, small = 0;
+  bool narrow = false;
   for (;; ++L) {
     const int cur = L % 3, old = (L + 2) % 3;
-    const unsigned long long* sc = step_counts(ws, cur, phase);
+    const unsigned long long* sc = step_counts<!Narrow>(ws, cur, phase);
     if constexpr (Hooked) {
       // a settle superstep ended at the barrier just passed: its duration
       if (s.id() == 0 && threadIdx.x == 0 && sst->open) {
@@ -537,13 +605,20 @@ __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const Gra
     }
     const bool dry = sc[0] == 0 && sc[1] == 0;
     const uint32_t sn = (uint32_t)sc[4], hn = (uint32_t)sc[5];
-    const bool unsettled = sn > sdone || hn > hdone;
+    const bool unsettled = !Narrow && (sn > sdone || hn > hdone);
     if (dry && !unsettled && (!ws.delta || sc[2] == 0)) break;
     if (leader) {
+      if (narrow) inner += max(ld_cg(&ws.cursor[old]), 1u) - 1u;
       ws.qcount[old] = 0;
       ws.hcount[old] = 0;
       ws.cursor[old] = 0;
       ws.hcursor[old] = 0;
+    }
+    if constexpr (Narrow) {
+      const bool fits = dry ? sc[2] <= (unsigned long long)s.P() * SsspDrain::kPile
+                            : sc[1] == 0 && sc[0] <= (unsigned long long)s.P() * ws.share;
+      small = fits ? small + 1 : 0;
+      narrow = fits && (small >= ws.patience || G.V <= (unsigned long long)s.P() * ws.share);
     }
     if (dry && unsettled) {
       // the bucket is settled: relax the heavy arcs of its vertices once,
@@ -572,7 +647,7 @@ __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const Gra
       hdone = hn;
       adone = an;
     } else if (dry) {
-      const uint32_t lo = split;
+      const uint32_t lo = split, fn = (uint32_t)sc[2];
       const unsigned long long nx = (unsigned long long)max(lo, (uint32_t)sc[3]) + ws.delta;
       split = (uint32_t)min(nx, 0xFFFFFFFFull);
       if (leader) {
@@ -580,8 +655,11 @@ __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const Gra
         ws.farcount[(phase + 2) % 3] = 0;
         ws.farmin[(phase + 2) % 3] = 0xFFFFFFFFu;
       }
-      far_filter(G, W, ws, L, phase, lo, split, (uint32_t)sc[2]);
+      if (narrow) sssp_narrow(G, ws, *drain, s.id(), s.P(), L, lo, split, phase + 1, true, fn, arcs);
+      else far_filter(G, W, ws, L, phase, lo, split, fn);
       ++phase;
+    } else if (narrow) {
+      sssp_narrow(G, ws, *drain, s.id(), s.P(), L, 0, split, phase, false, (uint32_t)sc[0], arcs);
     } else {
       sssp_sweep<true>(G, GH, W, ws, L, split, phase, pick(ws.q, L), (uint32_t)sc[0],
                        pick(ws.hc, L), (uint32_t)sc[1], 0u, whi, split_arcs, arcs);
@@ -595,7 +673,7 @@ __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const Gra
   for (int o = 16; o > 0; o >>= 1) arcs += __shfl_xor_sync(kFull, arcs, o);
   if (lane_id() == 0 && arcs) atomicAdd(&ws.stats[0], arcs);
   if (leader) {
-    ws.stats[1] = L;
+    ws.stats[1] = L + inner;
     ws.stats[2] = phase;
   }
 }
@@ -609,7 +687,7 @@ __global__ void __launch_bounds__(512, 2) k_sssp_xf(DiscoveryArgs a, GraphView G
   __shared__ uint32_t smin[512];
   if (!discover(a, &l)) return;
   XfSync s{&a, &l};
-  sssp_body<false>(s, G, GH, GT, ws, src, smin, nullptr);
+  sssp_body<false, false>(s, G, GH, GT, ws, src, smin, nullptr, nullptr);
 }
 
 __global__ void __launch_bounds__(512, 2) k_sssp_xf_sel(DiscoveryArgs a, GraphView G, GraphView GH,
@@ -619,14 +697,24 @@ __global__ void __launch_bounds__(512, 2) k_sssp_xf_sel(DiscoveryArgs a, GraphVi
   __shared__ SettleState sst;
   if (!discover(a, &l)) return;
   XfSync s{&a, &l};
-  sssp_body<true>(s, G, GH, GT, ws, src, smin, &sst);
+  sssp_body<true, false>(s, G, GH, GT, ws, src, smin, &sst, nullptr);
+}
+
+// Runs without the split that may take narrow supersteps (sssp_kernel).
+__global__ void __launch_bounds__(512, 2) k_sssp_xf_narrow(DiscoveryArgs a, GraphView G, GraphView, GraphView,
+                                                            SsspWs ws, uint32_t src) {
+  __shared__ LocalCtx l;
+  __shared__ SsspDrain drain;
+  if (!discover(a, &l)) return;
+  XfSync s{&a, &l};
+  sssp_body<false, true>(s, G, G, G, ws, src, nullptr, nullptr, &drain);
 }
 
 __global__ void __launch_bounds__(512, 2) k_sssp_grid(GraphView G, GraphView GH, GraphView GT,
                                                        SsspWs ws, uint32_t src) {
   __shared__ uint32_t smin[512];
   GridSync s;
-  sssp_body<false>(s, G, GH, GT, ws, src, smin, nullptr);
+  sssp_body<false, false>(s, G, GH, GT, ws, src, smin, nullptr, nullptr);
 }
 
 // Relaunch modes: an init launch, then one launch per superstep; the last
@@ -670,7 +758,7 @@ __global__ void __launch_bounds__(512, 3) k_sssp_glevel(GraphView G, SsspWs ws, 
   }
   const Warps W = warps_of(blockIdx.x, gridDim.x);
   unsigned long long arcs = 0;
-  const unsigned long long* sc = step_counts(ws, L % 3, 0);
+  const unsigned long long* sc = step_counts<false>(ws, L % 3, 0);
   sssp_sweep<false>(G, G, W, ws, L, 0xFFFFFFFFu, 0, pick(ws.q, L), (uint32_t)sc[0], pick(ws.hc, L),
                     (uint32_t)sc[1], 0u, kInf, false, arcs);
 #pragma unroll
@@ -946,6 +1034,9 @@ static size_t sssp_layout(const gdb_graph* g, char* base, uint32_t* d_dist, Sssp
   ws->trace = nullptr;
   ws->trace_cap = 0;
   ws->maxdeg = g->maxdeg;
+  ws->share = drain_share(g->E, V, SsspDrain::kCap);
+  // a graph of at most 8 arcs per vertex has no wide supersteps to wait for
+  ws->patience = g->maxdeg <= 8 ? 1u : 4u;
   ws->light = kInf;
   ws->qcap = V;
   ws->hcap = hcap;
@@ -1091,6 +1182,18 @@ static int settle_of(const gdb_ctx* c, uint32_t light, int force) {
   return c->opt.schedule == GDB_SCHED_LEARNED && c->d_mlp ? kSettleLearned : kSettleRule;
 }
 
+// The XF kernel of a run.  Narrow supersteps need whole arcs (no split) and
+// pay where frontiers are small for long: near-far runs, graphs of at most 8
+// arcs per vertex on average, and graphs whose every frontier is small.
+// What is left to k_sssp_xf besides the split is the plain worklist on
+// R-MAT-like graphs, a dozen wide supersteps that the narrow kernel's shared
+// memory slows (R-MAT-22 3.93 -> 4.0 to 4.1 ms per source).
+static auto sssp_kernel(const gdb_ctx* c, const gdb_graph* g, uint32_t delta, uint32_t light, int settle) {
+  const bool narrow = light >= kInf && (delta > 0 || g->E <= 8ull * g->V ||
+                                        g->V <= (uint64_t)c->sm_count * drain_share(g->E, g->V, SsspDrain::kCap));
+  return settle != kSettleRule ? k_sssp_xf_sel : narrow ? k_sssp_xf_narrow : k_sssp_xf;
+}
+
 int gdbi::sssp_enqueue(gdb_ctx* c, gdb_graph* g, void* wsbase, const uint32_t* d_srcs, uint32_t nsrc,
                        uint32_t* d_dist, cudaStream_t stream, const gdb::DiscoveryArgs& proto,
                        uint32_t delta, uint32_t light) {
@@ -1109,7 +1212,7 @@ int gdbi::sssp_enqueue(gdb_ctx* c, gdb_graph* g, void* wsbase, const uint32_t* d
   ws.mlp = c->d_mlp;
   GDB_CUDA(c, cudaMemsetAsync(cnt, 0, 512, stream));
   Shape s;
-  auto kx = ws.settle == kSettleRule ? k_sssp_xf : k_sssp_xf_sel;
+  auto kx = sssp_kernel(c, g, ws.delta, ws.light, ws.settle);
   int rc = persistent_shape(c, (const void*)kx, c->opt.block_size, 0, &s, false);
   if (rc) return rc;
   DiscoveryArgs a = proto;
@@ -1160,7 +1263,7 @@ static int sssp_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_sr
   c->last = gdb_run_stats{};
   if (xf) {
     Shape s;
-    auto kx = ws.settle == kSettleRule ? k_sssp_xf : k_sssp_xf_sel;
+    auto kx = sssp_kernel(c, g, ws.delta, ws.light, ws.settle);
     rc = persistent_shape(c, (const void*)kx, block, 0, &s, kind == GDB_BARRIER_XF);
     if (rc) return rc;
     DiscoveryArgs a = discovery_args(c, s);
@@ -1390,7 +1493,8 @@ int gdb_sssp_sources_device(gdb_ctx* c, gdb_graph* g, const uint32_t* d_sources,
   int rc = sssp_plan(c, g, 1, false, &delta, &relaunch, &light);
   if (rc) return rc;
   int occ = 0;
-  GDB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sssp_xf, c->opt.block_size, 0));
+  GDB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                  &occ, sssp_kernel(c, g, delta, light, settle_of(c, light, -1)), c->opt.block_size, 0));
   rc = run_on_lanes(c, n, kSsspLanes, true, sssp_workspace_bytes(g), occ * c->sm_count,
                     [&](gdb_lane& L, uint32_t i) {
     return sssp_enqueue(c, g, L.ws, d_sources + i, 1, d_dist + i * V, L.stream, lane_args(c, L),

@@ -123,11 +123,14 @@ typedef struct {
 } gdb_options;
 
 typedef struct {
-  uint32_t supersteps;       /* barrier intervals executed by the last run */
+  uint32_t supersteps;       /* supersteps of the last run: barrier intervals, where an
+                                interval in which CTAs relax several hops on their own
+                                counts the hops of the longest (BFS: its levels) */
   uint32_t participating;    /* CTAs that took part (discovered or launched) */
   uint32_t launched;         /* CTAs launched */
   uint32_t launches;         /* kernel launches by the last run */
-  uint64_t edges_processed;  /* arcs inspected (all passes) */
+  uint64_t edges_processed;  /* arcs inspected (all passes; a BFS level pushed counts
+                                its vertices' arcs once) */
   uint64_t work_units;       /* edges/s work unit of the last run */
   double kernel_ms;          /* device time of the last run (CUDA events) */
   uint32_t phases;           /* SSSP near-far phase changes of the last run */
