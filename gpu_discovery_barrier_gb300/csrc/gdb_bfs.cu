@@ -22,6 +22,7 @@
 //    level's features and duration with the mode fixed.
 #include <algorithm>
 
+#include "gdb_drain.cuh"
 #include "gdb_internal.h"
 #include "gdb_selector.cuh"
 
@@ -56,6 +57,12 @@ struct BfsWs {
   uint32_t* fbm;
   uint32_t fwords;             // ceil(V / 32) rounded up to a multiple of 4
   uint32_t swords;             // multiple of 4, <= fwords
+  // narrow tail (bfs_tail): two V-bit maps of the vertices queued for a
+  // superstep, by parity, in the bitmaps' space (nullptr: no tail); taken
+  // after `patience` levels in a row of at most `share` light vertices per
+  // CTA
+  uint32_t* queued;
+  uint32_t share, patience;
 };
 
 // Frontier bitmap slot of level L (nullptr without bitmaps).
@@ -363,9 +370,131 @@ __device__ __forceinline__ void bfs_bottom_up(const GraphView& G, const BfsWs& w
   qs.flush();
 }
 
+// The rest of a traversal whose frontiers have stayed small: buckets of
+// kTailLevels levels in narrow supersteps (gdb_drain.cuh).  Superstep S
+// starts from the queue of slot S, whose labels are at most `bound`.  Labels
+// are relaxed with atomicMin, so a vertex may be reached at too high a level
+// first and lowered later; the vertices reached at the bucket's last level
+// and those a CTA could not keep go to the next superstep's queue, once each
+// (their `queued` bit).  A queue too large for narrow supersteps, or with
+// heavy vertices, is relaxed one hop by the whole grid.
+// 4096^2 grid: from the corner (8,191 levels) 48.3 -> 12.2 ms, from the
+// middle 31.6 -> 6.4; 2530 x 40 13.7 -> 2.8; 64^2 0.66 -> 0.15.  What is left
+// is 1.5 us a level, a hop's two round trips.
+// kTailLevels 16 / 32 / 64 / 120: 13.8 / 12.7 / 12.2 / 12.0 ms (4096^2, corner).
+constexpr uint32_t kTailLevels = 64;
+using BfsDrain = DrainMem<448, 176>;
+static_assert(sizeof(BfsDrain) <= kStageWords * 4, "the slots take the staging buffers' place");
+
+template <class Sync>
+__device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
+                                      unsigned long long& arcs_out) {
+  const Warps W = warps_of(s.id(), s.P());
+  const bool leader = s.id() == 0 && threadIdx.x == 0;
+  const int lane = lane_id();
+  BfsDrain& m = *reinterpret_cast<BfsDrain*>(stage_mem());
+  const uint32_t first = bound;
+  unsigned long long walked = 0;
+  for (uint32_t i = W.gthread; i < 2 * ws.fwords; i += W.nthreads) ws.queued[i] = 0;
+  if (!s.sync()) return false;
+  for (;; ++S) {
+    const int cur = S % 3, nxt = (S + 1) % 3, old = (S + 2) % 3;
+    const unsigned long long* sc = cta_words<2>([&](unsigned long long* w) {
+      w[0] = ld_cg(&ws.qcount[cur]);
+      w[1] = ld_cg_u64(&ws.hcount[cur]);
+    });
+    const uint32_t n = (uint32_t)sc[0], nch = (uint32_t)sc[1];
+    if (n == 0 && nch == 0) break;
+    if (leader) {
+      ws.qcount[old] = 0;
+      ws.hcount[old] = 0;
+      ws.cursor[old] = 0;
+      ws.hcursor[old] = 0;
+    }
+    const Frontier out{pick(ws.q, S + 1), pick(ws.hc, S + 1), &ws.qcount[nxt], &ws.hcount[nxt],
+                       ws.qcap, ws.hcap, ws.overflow};
+    uint32_t* in_bits = ws.queued + (size_t)(S & 1) * ws.fwords;
+    uint32_t* out_bits = ws.queued + (size_t)((S + 1) & 1) * ws.fwords;
+    auto push = [&](bool want, uint32_t v) {
+      const uint32_t bit = 1u << (v & 31);
+      frontier_push(G, out, want && !(atomicOr(&out_bits[v >> 5], bit) & bit), v);
+    };
+    auto taken = [&](uint32_t v) {
+      atomicAnd(&in_bits[v >> 5], ~(1u << (v & 31)));
+      return ld_cg(&ws.dist[v]);
+    };
+    if (nch == 0 && n <= (unsigned long long)s.P() * ws.share) {
+      drain_reset(m);
+      drain_take(G, m, pick(ws.q, S), n, s.id(), s.P(), taken, push);
+      uint32_t fmin = 0;
+      drain_run(
+          G, m, bound + kTailLevels, fmin, walked, [](uint32_t) { return 1u; },
+          [&](uint32_t v) { return ld_cg(&ws.dist[v]); },
+          [&](uint32_t v, uint32_t d) { return atomicMin(&ws.dist[v], d); }, push, push);
+      bound += kTailLevels;
+    } else {
+      auto hop = [&](bool valid, uint32_t d, uint32_t arc) {
+        uint32_t v = 0;
+        bool want = false;
+        if (valid) {
+          v = __ldg(&G.col[arc]);
+          want = d < ld_cg(&ws.dist[v]) && d < atomicMin(&ws.dist[v], d);
+        }
+        push(want, v);
+      };
+      const uint32_t* q = pick(ws.q, S);
+      const uint4* hc = pick(ws.hc, S);
+      const uint32_t k = group_width(n, W.nwarps);
+      WorkTaker lt((n + k - 1) / k, W, &ws.cursor[cur]);
+      for (uint32_t g = lt.take(); g < lt.n; g = lt.take()) {
+        const uint32_t i = g * k + lane;
+        const bool act = (uint32_t)lane < k && i < n;
+        const uint32_t u = act ? ld_cg(&q[i]) : 0u;
+        const uint32_t d = act ? taken(u) + 1 : 0u;
+        group_arcs(G, act, u, [&](bool valid, int owner, uint32_t arc) {
+          hop(valid, __shfl_sync(kFull, d, owner), arc);
+        });
+      }
+      WorkTaker ht(nch, W, &ws.hcursor[cur], lt.n);
+      for (uint32_t c = ht.take(); c < nch; c = ht.take()) {
+        const uint4 ent = ld_cg(&hc[c]);
+        uint32_t b, e;
+        chunk_range(G, ent, b, e);
+        if (lane == 0 && ent.y == 0) taken(ent.x);
+        const uint32_t d = ld_cg(&ws.dist[ent.x]) + 1;
+        range_arcs(b, e, [&](bool valid, uint32_t arc) { hop(valid, d, arc); });
+      }
+      bound += 1;
+    }
+    if (!s.sync()) return false;
+  }
+  // levels of the traversal: one more than the largest; and the arcs of the
+  // vertices expanded here, each once (a vertex lowered after its expansion
+  // is walked again: seven arcs in 239,000 on a 300 x 200 grid)
+  uint32_t top = 0;
+  for (uint32_t v = W.gthread; v < G.V; v += W.nthreads) {
+    const uint32_t d = ld_cg(&ws.dist[v]);
+    if (d >= kInf) continue;
+    top = max(top, d + 1);
+    if (d >= first) arcs_out += __ldg(&G.row[v + 1]) - __ldg(&G.row[v]);
+  }
+  top = __reduce_max_sync(kFull, top);
+  if (lane == 0) atomicMax(&ws.stats[1], (unsigned long long)top);
+  return true;
+}
+
+// bfs_tail out of line, where its registers must not weigh on the levels'.
+template <class Sync>
+__device__ __noinline__ bool bfs_tail_call(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
+                                           unsigned long long& arcs_out) {
+  return bfs_tail(s, G, ws, S, bound, arcs_out);
+}
+
 // Hooked: the learned and forced-mode schedules (a decision inside every
 // barrier); a separate instantiation keeps the plain kernels' registers.
-template <bool Hooked, class Sync>
+// Tail: whether (kTailCall, kTailInline) the narrow tail may take over.
+enum { kTailNone = 0, kTailCall = 1, kTailInline = 2 };
+template <bool Hooked, int Tail, class Sync>
 __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t src,
                                          float* smlp, DecideState* dst, uint32_t* sbits) {
   const Warps W = warps_of(s.id(), s.P());
@@ -410,6 +539,8 @@ __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsW
   unsigned long long arcs = 0;
   uint32_t L = 0;
   bool bottom_up = false, prev_bottom_up = false;
+  uint32_t small = 0;  // levels in a row with a small frontier
+  bool tail = false;
   // direction-choice inputs, identical in every CTA: arcs of the frontier
   // (mf) and of the still-unvisited vertices (mu).  acc[k % 3] (stats[4..6])
   // collects the arcs of level k while level k-1 runs.
@@ -421,6 +552,18 @@ __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsW
     const uint32_t n = (uint32_t)sc[0];
     const unsigned long long hp = sc[1];
     if (n == 0 && hp == 0) break;
+    if constexpr (Tail != kTailNone) {
+      small = hp == 0 && n <= (unsigned long long)s.P() * ws.share ? small + 1 : 0;
+      if (ws.queued && small >= ws.patience) {
+        // the tail reads slot L's counts again; the slot after next is its to clear
+        bool done;
+        if constexpr (Tail == kTailCall) done = bfs_tail_call(s, G, ws, L, L, arcs);
+        else done = bfs_tail(s, G, ws, L, L, arcs);
+        if (!done) return;
+        tail = true;
+        break;
+      }
+    }
     if (ws.adaptive == kBfsHeuristic) {
       if (L > 0) {
         mf = sc[3];
@@ -460,7 +603,7 @@ __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsW
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(kFull, r, o);
   if (lane_id() == 0 && r) atomicAdd(&ws.stats[0], r);
-  if (leader) ws.stats[1] = L;
+  if (leader && !tail) ws.stats[1] = L;
 }
 
 // Dynamic shared memory of the traversal kernels: ws.swords words of the
@@ -470,13 +613,13 @@ __global__ void __launch_bounds__(512, 3) k_bfs_xf(DiscoveryArgs a, GraphView G,
   extern __shared__ uint4 bfs_stage[];
   if (!discover(a, &l)) return;
   XfSync s{&a, &l};
-  bfs_body<false>(s, G, ws, src, nullptr, nullptr, reinterpret_cast<uint32_t*>(bfs_stage));
+  bfs_body<false, kTailNone>(s, G, ws, src, nullptr, nullptr, reinterpret_cast<uint32_t*>(bfs_stage));
 }
 
 __global__ void __launch_bounds__(512, 3) k_bfs_grid(GraphView G, BfsWs ws, uint32_t src) {
   extern __shared__ uint4 bfs_stage[];
   GridSync s;
-  bfs_body<false>(s, G, ws, src, nullptr, nullptr, reinterpret_cast<uint32_t*>(bfs_stage));
+  bfs_body<false, kTailNone>(s, G, ws, src, nullptr, nullptr, reinterpret_cast<uint32_t*>(bfs_stage));
 }
 
 __global__ void __launch_bounds__(512, 3) k_bfs_xf_sel(DiscoveryArgs a, GraphView G, BfsWs ws,
@@ -487,7 +630,29 @@ __global__ void __launch_bounds__(512, 3) k_bfs_xf_sel(DiscoveryArgs a, GraphVie
   extern __shared__ uint4 bfs_stage[];
   if (!discover(a, &l)) return;
   XfSync s{&a, &l};
-  bfs_body<true>(s, G, ws, src, smlp, &dst, reinterpret_cast<uint32_t*>(bfs_stage));
+  bfs_body<true, kTailNone>(s, G, ws, src, smlp, &dst, reinterpret_cast<uint32_t*>(bfs_stage));
+}
+
+// The learned schedule of a traversal that has the GPU to itself.
+__global__ void __launch_bounds__(512, 3) k_bfs_xf_sel_tail(DiscoveryArgs a, GraphView G, BfsWs ws,
+                                                            uint32_t src) {
+  __shared__ LocalCtx l;
+  __shared__ float smlp[kParams];
+  __shared__ DecideState dst;
+  extern __shared__ uint4 bfs_stage[];
+  if (!discover(a, &l)) return;
+  XfSync s{&a, &l};
+  bfs_body<true, kTailCall>(s, G, ws, src, smlp, &dst, reinterpret_cast<uint32_t*>(bfs_stage));
+}
+
+// The plain and threshold schedules on graphs of few arcs per vertex, most
+// of whose levels are the tail's: registers for it.
+__global__ void __launch_bounds__(512, 2) k_bfs_xf_tail(DiscoveryArgs a, GraphView G, BfsWs ws, uint32_t src) {
+  __shared__ LocalCtx l;
+  extern __shared__ uint4 bfs_stage[];
+  if (!discover(a, &l)) return;
+  XfSync s{&a, &l};
+  bfs_body<false, kTailInline>(s, G, ws, src, nullptr, nullptr, reinterpret_cast<uint32_t*>(bfs_stage));
 }
 
 __global__ void __launch_bounds__(512, 3) k_bfs_grid_sel(GraphView G, BfsWs ws, uint32_t src) {
@@ -495,7 +660,7 @@ __global__ void __launch_bounds__(512, 3) k_bfs_grid_sel(GraphView G, BfsWs ws, 
   __shared__ DecideState dst;
   extern __shared__ uint4 bfs_stage[];
   GridSync s;
-  bfs_body<true>(s, G, ws, src, smlp, &dst, reinterpret_cast<uint32_t*>(bfs_stage));
+  bfs_body<true, kTailNone>(s, G, ws, src, smlp, &dst, reinterpret_cast<uint32_t*>(bfs_stage));
 }
 
 // Relaunch mode: init kernel, then one launch per level (no in-kernel barrier).
@@ -577,6 +742,17 @@ __global__ void __launch_bounds__(512, 3) k_bfs_glevel(GraphView G, BfsWs ws, ui
 
 using namespace gdbi;
 
+// Graphs whose vertices all have at most this many arcs run the
+// direction-optimising schedules as plain push.  A pull level scans every
+// unvisited vertex, a push level the frontier's arcs: with d <= 8 arcs per
+// vertex a pull can only pay once the unvisited vertices are fewer than
+// 8x the frontier, i.e. in the last few levels of a traversal, while the
+// per-level cost of the hooked kernel (the next frontier's degree loads,
+// the decision inside every barrier, the four-step batches) is paid on
+// every level: on the 4096^2 grid (8,191 levels) the learned BFS took
+// 91.9 ms against 51.0 ms push-only.
+constexpr uint32_t kPushOnlyMaxDeg = 8;
+
 // Words of one frontier bitmap slot of a graph of V vertices.
 static uint32_t bitmap_words(uint32_t V) { return ((V + 31) / 32 + 3) & ~3u; }
 
@@ -620,6 +796,10 @@ static size_t bfs_layout(const gdb_graph* g, char* base, uint32_t* d_dist, BfsWs
   ws->fbm = (uint32_t*)(base + o_fbm);
   ws->fwords = fwords;
   ws->swords = 0;
+  ws->queued = ws->fbm;
+  ws->share = drain_share(g->E, V, BfsDrain::kCap);
+  // a graph of few arcs per vertex has no wide levels to wait for
+  ws->patience = g->maxdeg <= kPushOnlyMaxDeg ? 1u : 8u;
   *cnt_out = cnt;
   return b.off;
 }
@@ -655,7 +835,8 @@ static void bfs_bitmap(gdb_ctx* c, const gdb_graph* g, BfsWs* ws, bool alone, si
 
 int gdbi::bfs_prepare(gdb_ctx* c) {
   // static + dynamic shared memory above 48 KB needs each kernel's opt-in
-  for (const void* k : {(const void*)k_bfs_xf, (const void*)k_bfs_xf_sel, (const void*)k_bfs_grid,
+  for (const void* k : {(const void*)k_bfs_xf, (const void*)k_bfs_xf_tail, (const void*)k_bfs_xf_sel, (const void*)k_bfs_xf_sel_tail,
+                        (const void*)k_bfs_grid,
                         (const void*)k_bfs_grid_sel})
     GDB_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageKbMax * 1024));
   return GDB_OK;
@@ -674,17 +855,6 @@ size_t gdbi::bfs_workspace_bytes(const gdb_graph* g) {
   return bfs_layout(g, nullptr, nullptr, nullptr, nullptr);
 }
 
-// Graphs whose vertices all have at most this many arcs run the
-// direction-optimising schedules as plain push.  A pull level scans every
-// unvisited vertex, a push level the frontier's arcs: with d <= 8 arcs per
-// vertex a pull can only pay once the unvisited vertices are fewer than
-// 8x the frontier, i.e. in the last few levels of a traversal, while the
-// per-level cost of the hooked kernel (the next frontier's degree loads,
-// the decision inside every barrier, the four-step batches) is paid on
-// every level: on the 4096^2 grid (8,191 levels) the learned BFS took
-// 91.9 ms against 51.0 ms push-only.
-constexpr uint32_t kPushOnlyMaxDeg = 8;
-
 // BfsWs::adaptive for c's schedule on g; the learned one needs a loaded
 // selector.
 static int bfs_mode(gdb_ctx* c, const gdb_graph* g, int* mode) {
@@ -697,6 +867,21 @@ static int bfs_mode(gdb_ctx* c, const gdb_graph* g, int* mode) {
     default: *mode = kBfsPlain; return GDB_OK;
   }
 }
+
+// The XF kernel of a run whose schedule is `mode` (BfsWs::adaptive).  The
+// narrow tail pays on long thin traversals and its code costs the levels'
+// loop registers (R-MAT, threshold schedule, one source: 0.270 -> 0.279 ms;
+// the learned kernel's levels run no slower with it, 0.301 -> 0.292, but on
+// lanes they do, 16 sources 2.85 -> 2.89 ms).  So it is there for graphs of
+// at most 8 arcs per vertex on average -- grids, meshes, roads; R-MAT graphs
+// have 16 and more -- and for learned traversals that have the GPU to
+// themselves, batches of uneven graphs among them.
+static const void* bfs_kernel(const gdb_graph* g, int mode, bool alone, bool tail) {
+  if (mode >= kBfsLearned) return tail && alone ? (const void*)k_bfs_xf_sel_tail : (const void*)k_bfs_xf_sel;
+  return tail && g->E <= 8ull * g->V ? (const void*)k_bfs_xf_tail : (const void*)k_bfs_xf;
+}
+
+using BfsKernel = void (*)(gdb::DiscoveryArgs, gdb::GraphView, BfsWs, uint32_t);
 
 // Enqueue one XF-barrier BFS (counter reset + persistent launch) on
 // `stream` without waiting, so that it can be stream-captured.  `proto`
@@ -715,15 +900,14 @@ int gdbi::bfs_enqueue(gdb_ctx* c, gdb_graph* g, void* wsbase, const uint32_t* d_
   if (c->opt.push_beta) ws.beta = c->opt.push_beta;
   GDB_CUDA(c, cudaMemsetAsync(cnt, 0, 512, stream));
   Shape s;
-  const bool sel = ws.adaptive >= kBfsLearned;
-  auto kx = sel ? k_bfs_xf_sel : k_bfs_xf;
+  const void* kx = bfs_kernel(g, ws.adaptive, alone, true);
   size_t smem = 0;
   bfs_bitmap(c, g, &ws, alone, &smem);
-  rc = persistent_shape(c, (const void*)kx, c->opt.block_size, smem, &s, false);
+  rc = persistent_shape(c, kx, c->opt.block_size, smem, &s, false);
   if (rc) return rc;
   DiscoveryArgs a = proto;
   a.expected = std::min(s.grid, s.fit);
-  kx<<<s.grid, c->opt.block_size, smem, stream>>>(a, g->view(), ws, 0u);
+  ((BfsKernel)kx)<<<s.grid, c->opt.block_size, smem, stream>>>(a, g->view(), ws, 0u);
   GDB_CUDA(c, cudaGetLastError());
   return GDB_OK;
 }
@@ -741,6 +925,7 @@ static int bfs_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_src
   bfs_layout(g, base, d_dist, &ws, &cnt);
   if (force >= 0) {
     ws.adaptive = force;
+    ws.queued = nullptr;  // traces record every level
   } else {
     int rc0 = bfs_mode(c, g, &ws.adaptive);
     if (rc0) return rc0;
@@ -763,14 +948,14 @@ static int bfs_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_src
   int rc = GDB_OK;
   if (kind == GDB_BARRIER_XF || kind == GDB_BARRIER_XF_FIXED) {
     Shape s;
-    auto kx = ws.adaptive >= kBfsLearned ? k_bfs_xf_sel : k_bfs_xf;
+    const void* kx = bfs_kernel(g, ws.adaptive, true, ws.queued != nullptr);
     size_t smem = 0;
     bfs_bitmap(c, g, &ws, true, &smem);
-    rc = persistent_shape(c, (const void*)kx, block, smem, &s, kind == GDB_BARRIER_XF);
+    rc = persistent_shape(c, kx, block, smem, &s, kind == GDB_BARRIER_XF);
     if (rc) return rc;
     DiscoveryArgs a = discovery_args(c, s);
     GDB_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    kx<<<s.grid, block, smem, c->stream>>>(a, G, ws, src);
+    ((BfsKernel)kx)<<<s.grid, block, smem, c->stream>>>(a, G, ws, src);
     GDB_CUDA(c, cudaGetLastError());
     GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     rc = finish_run(c);
@@ -904,7 +1089,7 @@ int gdb_bfs_sources_device(gdb_ctx* c, gdb_graph* g, const uint32_t* d_sources, 
   int rc = bfs_mode(c, g, &mode);
   if (rc) return rc;
   int occ = 0;
-  const void* kx = mode >= kBfsLearned ? (const void*)k_bfs_xf_sel : (const void*)k_bfs_xf;
+  const void* kx = bfs_kernel(g, mode, false, true);
   const size_t smem = (size_t)bitmap_stage_words(c, mode, g->V, false) * 4;
   GDB_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kx, c->opt.block_size, smem));
   const int fit = occ * c->sm_count;
@@ -1122,6 +1307,9 @@ extern "C" int gdb_bfs_noalloc(const uint32_t* d_row_ptr, const uint32_t* d_col,
   ws.srcs = nullptr;
   ws.nsrc = 0;
   ws.fbm = nullptr;  // plain push: no frontier bitmaps
+  ws.queued = nullptr;  // and no room for the tail's bits
+  ws.share = 0;
+  ws.patience = 0;
   ws.fwords = 0;
   ws.swords = 0;
   DiscoveryArgs a;

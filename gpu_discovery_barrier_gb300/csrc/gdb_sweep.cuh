@@ -374,9 +374,14 @@ struct WarpStage {
 // This warp's 64-slot staging buffer number k (0-2), shared by the
 // staged queues of a superstep.
 __device__ __forceinline__ uint32_t* warp_stage(int k) {
-  __shared__ uint32_t buf[3][kMaxGraphWarps][64];
+  __shared__ __align__(16) uint32_t buf[3][kMaxGraphWarps][64];
   return buf[k][threadIdx.x >> 5];
 }
+
+// The staging buffers as one block of shared memory, for supersteps that
+// stage no pushes.
+constexpr uint32_t kStageWords = 3 * kMaxGraphWarps * 64;
+__device__ __forceinline__ uint32_t* stage_mem() { return warp_stage(0) - (threadIdx.x >> 5) * 64; }
 
 // A staged frontier: light entries through the warp's buffer k.
 __device__ __forceinline__ WarpStage frontier_stage(const Frontier& F, int k) {
