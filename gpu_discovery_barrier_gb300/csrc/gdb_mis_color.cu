@@ -4,7 +4,8 @@
 // per round every undecided vertex takes the minimum priority over its
 // undecided neighbours (mis1, :245-270); undecided strict local minima join
 // the set, s = 2, and mark their undecided neighbours decided (mis2,
-// :277-312).  The reference stages neighbour marks in cu[] and commits them
+// :277-312).  What decides is whether some undecided neighbour is at or
+// below the vertex's own priority, so a vertex here stops at the first.  The reference stages neighbour marks in cu[] and commits them
 // in a third barrier interval (mis3, :322-330); here the marks go straight
 // into the state array -- two winners are never adjacent, so no winner test
 // can see a mark of the same round -- and a round needs two barriers.
@@ -33,22 +34,21 @@ struct MisWs {
   int32_t* state;       // -1 undecided, -2 decided
   uint32_t* ukey;       // the priority key while undecided, kMisGone once decided
   int32_t* s;           // output: 2 in the set, 0 otherwise
-  uint32_t* mn;         // light vertices: key of the min undecided neighbour priority
-  uint32_t* hmn[2];     // heavy vertices, by heavy index, double-buffered by round
+  uint32_t* u[2];       // light vertices undecided when a round starts, by round parity (round 0: all)
+  uint32_t* wq;         // the round's light winners
+  uint32_t* hlost;      // heavy vertices, by heavy index: 1 + the last round they lost
   const float* prio;
-  uint32_t* cursor;     // [3]
-  uint32_t* hcursor;    // [3]
-  uint32_t* flag;       // [3] some vertex undecided
-  uint32_t* won;        // [3] some vertex joined the set (mis2 supersteps)
+  uint32_t* ucount;     // [3] by round % 3
+  uint32_t* wcount;     // [3]
+  uint32_t* flag;       // [3] some vertex undecided: bit 0 light, bit 1 heavy
+  uint32_t* won;        // [3] some heavy vertex joined the set
   int* stuck;           // set when a round chose no vertex (see mis_body)
   unsigned long long* stats;  // [0] arcs, [1] rounds
 };
 
-constexpr uint32_t kMisNone = 0xFFFFFFFFu;  // no arc in this lane's step
-// ukey of a decided vertex: above every key mis1 can take as a minimum
-// (BIGNUM's key and all finite priorities), so a decided neighbour never
-// lowers one, and mis1 needs one load per neighbour instead of the state
-// and then the priority
+// ukey of a decided vertex: above every key below BIGNUM's, so a decided
+// neighbour never beats an undecided vertex, and mis1 needs one load per
+// neighbour instead of the state and then the priority
 constexpr uint32_t kMisGone = 0xFFFFFFFFu;
 
 // A priority's key: fkey's order, with every NaN, of either sign, at
@@ -60,167 +60,229 @@ __device__ __forceinline__ uint32_t mis_key(float f) { return isnan(f) ? kMisGon
 
 // mis_kernel.cl:78-93 (init), run by every thread of the grid.
 __device__ __forceinline__ void mis_init(const GraphView& G, const Warps& W, const MisWs& ws, bool leader) {
-  const uint32_t big = fkey(kMisBig);
   for (uint32_t v = W.gthread; v < G.V; v += W.nthreads) {
     ws.state[v] = -1;
     ws.s[v] = 0;
     ws.ukey[v] = mis_key(__ldg(&ws.prio[v]));
   }
-  for (uint32_t h = W.gthread; h < G.nheavy; h += W.nthreads) ws.hmn[0][h] = ws.hmn[1][h] = big;
+  for (uint32_t h = W.gthread; h < G.nheavy; h += W.nthreads) ws.hlost[h] = 0;
   if (leader) {
-    for (int i = 0; i < 3; ++i) ws.cursor[i] = ws.hcursor[i] = ws.flag[i] = ws.won[i] = 0;
+    for (int i = 0; i < 3; ++i) ws.ucount[i] = ws.wcount[i] = ws.flag[i] = ws.won[i] = 0;
     *ws.stuck = 0;
     ws.stats[0] = ws.stats[1] = 0;
   }
 }
 
-// mis1 of round r (superstep t): every undecided vertex takes the minimum
-// priority key over its undecided neighbours; flag[t % 3] records whether
-// any vertex was still undecided.  Every thread of the grid calls it.
-__device__ __forceinline__ void mis_phase1(const GraphView& G, const MisWs& ws, uint32_t r, uint32_t t,
-                                           uint32_t* my, bool leader, unsigned long long& arcs) {
-  const int lane = lane_id();
-  const uint32_t big = fkey(kMisBig);
-  // flag[t % 3] is read after this superstep's barrier: clear the slot
-  // of superstep t - 2
-  const int cur = t % 3, old = (t + 1) % 3;
-  if (leader) ws.cursor[old] = ws.hcursor[old] = ws.flag[old] = 0;
-  bool undecided_seen = false;
-  // four 32-arc steps at once: the column and key loads of the four are
-  // in flight together
-  sweep_light4(
-      G, &ws.cursor[cur],
-      [&](uint32_t v, bool in_range) {
-        const bool und = in_range && ld_cg(&ws.state[v]) == -1;
-        my[lane] = big;
-        undecided_seen |= und;
-        return und;
-      },
-      [&](const bool* valid, const int* owner, const uint32_t* arc) {
-        uint32_t u[4], k[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          u[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
-          arcs += valid[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) k[j] = valid[j] ? ld_cg(&ws.ukey[u[j]]) : kMisGone;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (k[j] < my[owner[j]]) atomicMin(&my[owner[j]], k[j]);
-      },
-      [&](uint32_t v, bool act) {
-        if (act) ws.mn[v] = my[lane];
-      });
-  uint32_t* hmn = pick(ws.hmn, r);
-  sweep_heavy(G, &ws.hcursor[cur], [&](uint32_t v, uint32_t h, uint32_t, uint32_t b, uint32_t e) {
-    // a heavy winner's own state is settled here (see mis2)
-    if (ld_cg(&ws.s[v]) == 2) {
-      if (lane == 0) {
-        ws.state[v] = -2;
-        ws.ukey[v] = kMisGone;
-      }
-      return;
-    }
-    if (ld_cg(&ws.state[v]) != -1) return;
-    undecided_seen = true;
-    uint32_t m = big;
-    // a chunk (kChunk = 128 arcs) as four steps with their loads in flight
-    uint32_t u[4], k[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t a = b + 32 * j + lane;
-      u[j] = a < e ? __ldg(&G.col[a]) : kMisNone;
-      arcs += a < e;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) k[j] = u[j] != kMisNone ? ld_cg(&ws.ukey[u[j]]) : kMisGone;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m = min(m, k[j]);
-    m = warp_min_u32(m);
-    if (lane == 0 && m < big) atomicMin(&hmn[h], m);
-  });
-  cta_or(undecided_seen, &ws.flag[cur], 1u);
+// The warp's 32 chunk entries from `base`, one per lane; past the table's
+// end: no entry (w = 0 chunks).
+__device__ __forceinline__ uint4 mis_chunk(const GraphView& G, uint32_t base) {
+  const uint32_t c = base + lane_id();
+  return c < G.nheavy_chunks ? __ldg(&G.heavy_chunk[c]) : make_uint4(0, 0, 0, 0);
 }
 
-// mis2 of round r (superstep t): strict local minima join the set and
-// decide their neighbours.  Every thread of the grid calls it.
-__device__ __forceinline__ void mis_phase2(const GraphView& G, const Warps& W, const MisWs& ws, uint32_t r,
-                                           uint32_t t, bool leader, unsigned long long& arcs) {
+// mis1 of round r: an undecided vertex with an undecided neighbour at or
+// below its own key loses the round; the light ones of the others go to the
+// winners' queue, the losers to the next round's list.  Every thread of the
+// grid calls it.
+//
+// A vertex of random priority meets a neighbour that beats it after a few
+// arcs, where the minimum over all of them read 128 M columns and keys in
+// round 0 (R-MAT-22): each lane probes up to kMisProbe arcs of its own
+// vertex, the warp scans what is left of the lists that go on, 128 arcs at
+// a time, and a heavy vertex's chunks stop at the first that finds one.
+// The keys do not change during mis1: ordinary loads, through L1.
+//   R-MAT-22: 2.99 -> 0.68 ms; 4,097 to 1,500,000 vertices 1.6 to 2.2 times
+// (kMisProbe 4 / 8 / 16 / 32: 0.69 / 0.68 / 0.67 / 0.69).
+constexpr uint32_t kMisProbe = 8;
+
+__device__ __forceinline__ void mis_phase1(const GraphView& G, const Warps& W, const MisWs& ws, uint32_t r,
+                                           bool leader, unsigned long long& arcs) {
   const int lane = lane_id();
   const uint32_t big = fkey(kMisBig);
-  // flag[t % 3] and won[t % 3] are read after this superstep's barrier:
-  // clear the slots of superstep t - 2
-  const int cur = t % 3, old = (t + 1) % 3;
-  if (leader) ws.cursor[old] = ws.hcursor[old] = ws.flag[old] = ws.won[old] = 0;
-  bool any_win = false;
-  // next round's heavy minima start from BIGNUM
-  for (uint32_t h = W.gthread; h < G.nheavy; h += W.nthreads) pick(ws.hmn, r + 1)[h] = big;
-  sweep_light4(
-      G, &ws.cursor[cur],
-      [&](uint32_t v, bool in_range) {
-        bool win = false;
-        if (in_range && ld_cg(&ws.state[v]) == -1 && mis_key(__ldg(&ws.prio[v])) < ws.mn[v]) {
-          win = true;
-          any_win = true;
-          ws.s[v] = 2;
-          ws.state[v] = -2;
-          ws.ukey[v] = kMisGone;
-        }
-        return win;
-      },
-      [&](const bool* valid, const int*, const uint32_t* arc) {
+  const uint32_t cur = r % 3, nxt = (r + 1) % 3, old = (r + 2) % 3;
+  // slots last read in round r - 1 (the list) and r - 2 (the rest)
+  const unsigned long long* w = cta_words<2>([&](unsigned long long* x) {
+    x[0] = r == 0 ? G.V : ld_cg(&ws.ucount[cur]);
+    x[1] = r == 0 ? 2u : ld_cg(&ws.flag[old]) & 2u;  // heavy vertices left by round r - 1
+  });
+  const uint32_t n = (uint32_t)w[0];
+  const bool heavy = w[1] != 0;
+  if (leader) ws.ucount[old] = ws.wcount[nxt] = ws.flag[nxt] = ws.won[nxt] = 0;
+  const uint32_t* list = pick(ws.u, r);
+  WarpStage lose{warp_stage(0), pick(ws.u, r + 1), &ws.ucount[nxt], G.V, ws.stuck};
+  WarpStage win{warp_stage(1), ws.wq, &ws.wcount[cur], G.V, ws.stuck};
+  bool seen = false, seen_heavy = false;
+  for (uint32_t g = W.gwarp; g * 32 < n; g += W.nwarps) {
+    const uint32_t i = g * 32 + lane;
+    const uint32_t v = i < n ? (r == 0 ? i : ld_cg(&list[i])) : 0u;
+    const bool act = i < n && (r == 0 ? !is_heavy(G, v) : ld_cg(&ws.state[v]) == -1);
+    bool lost = false;
+    uint32_t b = 0, e = 0, kv = 0;
+    if (act) {
+      b = __ldg(&G.row[v]);
+      e = __ldg(&G.row[v + 1]);
+      kv = ws.ukey[v];
+      lost = kv >= big;  // BIGNUM and above never win
+      const uint32_t stop = min(e, b + kMisProbe);
+      for (; b < stop && !lost; b += 4) {
         uint32_t u[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          u[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
-          arcs += valid[j];
-        }
+        for (int j = 0; j < 4; ++j) u[j] = b + j < stop ? __ldg(&G.col[b + j]) : 0u;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (valid[j] && ld_cg(&ws.state[u[j]]) == -1) {
-            ws.state[u[j]] = -2;
-            ws.ukey[u[j]] = kMisGone;
+        for (int j = 0; j < 4; ++j) {
+          if (b + j < stop) {
+            ++arcs;
+            lost = lost || ws.ukey[u[j]] <= kv;
           }
-      },
-      [](uint32_t, bool) {});
-  const uint32_t* hmn = pick(ws.hmn, r);
+        }
+      }
+    }
+    for (unsigned m = __ballot_sync(kFull, act && !lost && b < e); m; m &= m - 1) {
+      const int o = __ffs(m) - 1;
+      const uint32_t bb = __shfl_sync(kFull, b, o), ee = __shfl_sync(kFull, e, o);
+      const uint32_t kk = __shfl_sync(kFull, kv, o);
+      uint32_t u[4], low = kMisGone;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t a = bb + 32 * j + lane;
+        u[j] = a < ee ? __ldg(&G.col[a]) : kMisGone;
+        arcs += a < ee;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (u[j] != kMisGone) low = min(low, ws.ukey[u[j]]);
+      // at most kHeavyDeg arcs: one step
+      if (__any_sync(kFull, low <= kk) && lane == o) lost = true;
+    }
+    seen |= act;
+    win.add(act && !lost, v);
+    lose.add(act && lost, v);
+  }
+  win.flush();
+  lose.flush();
+  for (uint32_t base = W.gwarp * 32; heavy && base < G.nheavy_chunks; base += W.nwarps * 32) {
+    const uint4 ent = mis_chunk(G, base);
+    bool todo = ent.w != 0 && ld_cg(&ws.state[ent.x]) == -1;
+    if (todo && ld_cg(&ws.s[ent.x]) == 2) {
+      // a heavy winner's own state is settled here (see mis2)
+      if (ent.y == 0) {
+        ws.state[ent.x] = -2;
+        ws.ukey[ent.x] = kMisGone;
+      }
+      todo = false;
+    }
+    seen_heavy |= todo;
+    uint32_t kv = 0, rb = 0, re = 0;
+    if (todo) {
+      kv = ws.ukey[ent.x];
+      rb = __ldg(&G.row[ent.x]) + ent.y * kChunk;
+      re = min(__ldg(&G.row[ent.x + 1]), rb + kChunk);
+      if (kv >= big) {
+        ws.hlost[ent.z] = r + 1;
+        todo = false;
+      }
+    }
+    for (unsigned m = __ballot_sync(kFull, todo); m;) {
+      const int o = __ffs(m) - 1;
+      const uint32_t h = __shfl_sync(kFull, ent.z, o), kk = __shfl_sync(kFull, kv, o);
+      const uint32_t bb = __shfl_sync(kFull, rb, o), ee = __shfl_sync(kFull, re, o);
+      const bool lost = ld_cg(&ws.hlost[h]) == r + 1;  // by another chunk, in flight with the columns
+      uint32_t u[4], low = kMisGone;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t a = bb + 32 * j + lane;
+        u[j] = a < ee ? __ldg(&G.col[a]) : kMisGone;
+      }
+      if (!lost) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          arcs += u[j] != kMisGone;
+          if (u[j] != kMisGone) low = min(low, ws.ukey[u[j]]);
+        }
+      }
+      const bool beaten = __any_sync(kFull, !lost && low <= kk);
+      if (beaten && lane == 0) ws.hlost[h] = r + 1;
+      m &= beaten || __any_sync(kFull, lost) ? ~__ballot_sync(kFull, ent.w != 0 && ent.z == h) : m - 1;
+    }
+  }
+  cta_or(seen, &ws.flag[cur], 1u);
+  cta_or(seen_heavy, &ws.flag[cur], 2u);
+}
+
+// mis2 of round r: the winners join the set and decide their neighbours.
+// Every thread of the grid calls it.
+__device__ __forceinline__ void mis_phase2(const GraphView& G, const Warps& W, const MisWs& ws, uint32_t r,
+                                           unsigned long long& arcs) {
+  const int lane = lane_id();
+  const uint32_t cur = r % 3;
+  const unsigned long long* w = cta_words<2>([&](unsigned long long* x) {
+    x[0] = ld_cg(&ws.wcount[cur]);
+    x[1] = ld_cg(&ws.flag[cur]) & 2u;
+  });
+  const uint32_t n = (uint32_t)w[0];
+  const bool heavy = w[1] != 0;
+  auto decide = [&](const bool* valid, const uint32_t* arc) {
+    uint32_t u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      u[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
+      arcs += valid[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (valid[j] && ld_cg(&ws.state[u[j]]) == -1) {
+        ws.state[u[j]] = -2;
+        ws.ukey[u[j]] = kMisGone;
+      }
+  };
+  const uint32_t k = group_width(n, W.nwarps);
+  for (uint32_t g = W.gwarp; g * k < n; g += W.nwarps) {
+    const uint32_t i = g * k + lane;
+    const bool act = (uint32_t)lane < k && i < n;
+    const uint32_t v = act ? ld_cg(&ws.wq[i]) : 0u;
+    if (act) {
+      ws.s[v] = 2;
+      ws.state[v] = -2;
+      ws.ukey[v] = kMisGone;
+    }
+    group_arcs4(G, act, v, [&](const bool* valid, const int*, const uint32_t* arc) { decide(valid, arc); });
+  }
   // A heavy winner is split over chunks: its own state stays -1 here so
   // every chunk sees the same test; s = 2 marks it and mis1 of the next
   // round settles its state (all its neighbours are decided by then, so
   // nobody reads it in between).
-  sweep_heavy(G, &ws.hcursor[cur], [&](uint32_t v, uint32_t h, uint32_t, uint32_t b, uint32_t e) {
-    if (ld_cg(&ws.state[v]) != -1) return;
-    if (!(mis_key(__ldg(&ws.prio[v])) < ld_cg(&hmn[h]))) return;
-    any_win = true;
-    if (lane == 0) ws.s[v] = 2;
-    uint32_t u[4];
+  bool any_win = false;
+  for (uint32_t base = W.gwarp * 32; heavy && base < G.nheavy_chunks; base += W.nwarps * 32) {
+    const uint4 ent = mis_chunk(G, base);
+    const bool won = ent.w != 0 && ld_cg(&ws.state[ent.x]) == -1 && ld_cg(&ws.hlost[ent.z]) != r + 1;
+    any_win |= won;
+    if (won && ent.y == 0) ws.s[ent.x] = 2;
+    for (unsigned m = __ballot_sync(kFull, won); m; m &= m - 1) {
+      const int o = __ffs(m) - 1;
+      const uint4 x = make_uint4(__shfl_sync(kFull, ent.x, o), __shfl_sync(kFull, ent.y, o), 0u, 0u);
+      uint32_t b, e;
+      chunk_range(G, x, b, e);
+      bool valid[4];
+      uint32_t arc[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t a = b + 32 * j + lane;
-      u[j] = a < e ? __ldg(&G.col[a]) : kMisNone;
-      arcs += a < e;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (u[j] != kMisNone && ld_cg(&ws.state[u[j]]) == -1) {
-        ws.state[u[j]] = -2;
-        ws.ukey[u[j]] = kMisGone;
+      for (int j = 0; j < 4; ++j) {
+        arc[j] = b + 32 * j + lane;
+        valid[j] = arc[j] < e;
       }
-  });
+      decide(valid, arc);
+    }
+  }
   cta_or(any_win, &ws.won[cur], 1u);
 }
 
 template <class Sync>
-__device__ __forceinline__ void mis_body(Sync& s, const GraphView& G, const MisWs& ws, uint32_t* smem) {
+__device__ __forceinline__ void mis_body(Sync& s, const GraphView& G, const MisWs& ws) {
   const Warps W = warps_of(s.id(), s.P());
   const bool leader = s.id() == 0 && threadIdx.x == 0;
-  uint32_t* my = smem + (threadIdx.x & ~31u);
   mis_init(G, W, ws, leader);
   if (!s.sync()) return;
   unsigned long long arcs = 0;
   uint32_t r = 0;
-  uint32_t t = 0;  // cursor slot counter: two sweeps per round
   // A round in which no vertex joins the set changes nothing, so every
   // later round would repeat it: adjacent vertices of equal priority, NaN
   // priorities and priorities of BIGNUM and above never win.  The
@@ -229,16 +291,13 @@ __device__ __forceinline__ void mis_body(Sync& s, const GraphView& G, const MisW
   // least that one, so V rounds always suffice: the bound below holds the
   // loop to them whatever happens.
   for (; r <= G.V; ++r) {
-    mis_phase1(G, ws, r, t, my, leader, arcs);
+    const uint32_t cur = r % 3;
+    mis_phase1(G, W, ws, r, leader, arcs);
     if (!s.sync()) return;
-    const int cur = t % 3;
-    ++t;
     if (cta_words<1>([&](unsigned long long* w) { w[0] = ld_cg(&ws.flag[cur]); })[0] == 0) break;
-    mis_phase2(G, W, ws, r, t, leader, arcs);
+    mis_phase2(G, W, ws, r, arcs);
     if (!s.sync()) return;
-    const int cur2 = t % 3;
-    ++t;
-    if (cta_words<1>([&](unsigned long long* w) { w[0] = ld_cg(&ws.won[cur2]); })[0] == 0) {
+    if (cta_words<1>([&](unsigned long long* w) { w[0] = ld_cg(&ws.won[cur]) | ld_cg(&ws.wcount[cur]); })[0] == 0) {
       if (leader) *ws.stuck = 1;
       break;
     }
@@ -252,42 +311,39 @@ __device__ __forceinline__ void mis_body(Sync& s, const GraphView& G, const MisW
 
 __global__ void __launch_bounds__(512, 3) k_mis_xf(DiscoveryArgs a, GraphView G, MisWs ws) {
   __shared__ LocalCtx l;
-  __shared__ uint32_t smem[1024];
   if (!discover(a, &l)) return;
   XfSync s{&a, &l};
-  mis_body(s, G, ws, smem);
+  mis_body(s, G, ws);
 }
 
 // Relaunch form (mis.cpp:314-364: one launch per phase, the stop flag read
-// back after each): control state s[0] = round, s[1] = superstep, s[2] =
-// phase (1: mis1, 2: mis2).
+// back after each): control state s[0] = round, s[2] = phase (1: mis1, 2:
+// mis2).
 __global__ void k_mis_rl_init(GraphView G, MisWs ws) {
   mis_init(G, warps_of(blockIdx.x, gridDim.x), ws, blockIdx.x == 0 && threadIdx.x == 0);
 }
 
 __global__ void __launch_bounds__(512, 3) k_mis_rl_step(GraphView G, MisWs ws, StepCtl* ctl,
                                                        cudaGraphConditionalHandle cond) {
-  __shared__ uint32_t smem[1024];
   const StepCtl& st0 = step_state(ctl);
-  const uint32_t r = st0.s[0], t = st0.s[1], phase = st0.s[2];
-  const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+  const uint32_t r = st0.s[0], phase = st0.s[2];
+  const Warps W = warps_of(blockIdx.x, gridDim.x);
   unsigned long long arcs = 0;
   if (phase == 1)
-    mis_phase1(G, ws, r, t, smem + (threadIdx.x & ~31u), leader, arcs);
+    mis_phase1(G, W, ws, r, blockIdx.x == 0 && threadIdx.x == 0, arcs);
   else
-    mis_phase2(G, warps_of(blockIdx.x, gridDim.x), ws, r, t, leader, arcs);
+    mis_phase2(G, W, ws, r, arcs);
   arcs = warp_add_u64(arcs);
   if (lane_id() == 0 && arcs) atomicAdd(&ws.stats[0], arcs);
   step_end(ctl, cond, [&](StepCtl& st) {
-    st.s[1] = t + 1;
     if (phase == 1) {
-      if (__ldcg(&ws.flag[t % 3]) == 0) {
+      if (__ldcg(&ws.flag[r % 3]) == 0) {
         ws.stats[1] = r + 1;
         return false;
       }
       st.s[2] = 2;
     } else {
-      if (__ldcg(&ws.won[t % 3]) == 0) {
+      if ((__ldcg(&ws.won[r % 3]) | __ldcg(&ws.wcount[r % 3])) == 0) {
         // no vertex joined the set: every later round would repeat this one
         *ws.stuck = 1;
         ws.stats[1] = r + 1;
@@ -811,9 +867,10 @@ static int mis_run(gdb_ctx* c, gdb_graph* g, const float* d_prio, int32_t* d_s) 
   if (!graph_ok(c, g) || !d_prio || !d_s) return GDB_ERR_INVALID;
   const uint32_t hcap = std::max<uint32_t>(g->nheavy, 1);
   Bump b;
-  const size_t o_state = b.take((size_t)g->V * 4), o_mn = b.take((size_t)g->V * 4);
-  const size_t o_ukey = b.take((size_t)g->V * 4);
-  const size_t o_h0 = b.take(hcap * 4), o_h1 = b.take(hcap * 4), o_cnt = b.take(256);
+  const size_t o_state = b.take((size_t)g->V * 4), o_ukey = b.take((size_t)g->V * 4);
+  const size_t o_u0 = b.take((size_t)g->V * 4), o_u1 = b.take((size_t)g->V * 4);
+  const size_t o_wq = b.take((size_t)g->V * 4);
+  const size_t o_h = b.take(hcap * 4), o_cnt = b.take(256);
   const size_t o_ctl = b.take(sizeof(StepCtl));
   char* base = (char*)workspace(c, b.off);
   if (!base) return GDB_ERR_OOM;
@@ -821,14 +878,15 @@ static int mis_run(gdb_ctx* c, gdb_graph* g, const float* d_prio, int32_t* d_s) 
   ws.state = (int32_t*)(base + o_state);
   ws.ukey = (uint32_t*)(base + o_ukey);
   ws.s = d_s;
-  ws.mn = (uint32_t*)(base + o_mn);
-  ws.hmn[0] = (uint32_t*)(base + o_h0);
-  ws.hmn[1] = (uint32_t*)(base + o_h1);
+  ws.u[0] = (uint32_t*)(base + o_u0);
+  ws.u[1] = (uint32_t*)(base + o_u1);
+  ws.wq = (uint32_t*)(base + o_wq);
+  ws.hlost = (uint32_t*)(base + o_h);
   ws.prio = d_prio;
   char* cnt = base + o_cnt;
   ws.stats = (unsigned long long*)cnt;
-  ws.cursor = (uint32_t*)(cnt + 64);
-  ws.hcursor = (uint32_t*)(cnt + 80);
+  ws.ucount = (uint32_t*)(cnt + 64);
+  ws.wcount = (uint32_t*)(cnt + 80);
   ws.flag = (uint32_t*)(cnt + 96);
   ws.won = (uint32_t*)(cnt + 112);
   ws.stuck = (int*)(cnt + 128);
