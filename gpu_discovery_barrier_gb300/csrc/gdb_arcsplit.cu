@@ -11,7 +11,7 @@
 // Everything is built on the device: per-vertex class counts (a warp per
 // vertex of degree <= 128, a CTA per heavier vertex), exclusive scans into
 // the two row arrays, an order-preserving scatter (ballot compaction), and
-// the heavy tables from scans of the halves' degrees.  Only totals come
+// the heavy tables from the halves' degrees.  Only totals come
 // back to the host.  The partition is cached on the graph per bound and
 // dropped when its weights change.
 #include <algorithm>
@@ -295,38 +295,108 @@ __global__ void k_transpose(GraphView H, const uint32_t* rt, uint32_t* fill, uin
   }
 }
 
-// Heavy-vertex marks of a CSR given by its row array: flag (degree >
-// kHeavyDeg), chunk count, the membership bitmap and the largest degree.
-__global__ void k_heavy_marks(const uint32_t* row, uint32_t V, uint32_t* flag, uint32_t* nch,
+// Heavy-vertex table of a CSR given by its row array, in tiles of 1,024
+// consecutive vertices: the tiles' counts (heavy vertices << 32 | chunks)
+// with the membership bitmap and the largest degree, a scan over the tiles,
+// and the entries from each tile's start.  R-MAT-22: graph creation over
+// device arrays (this, 82 us, and the CSR check, 115) 0.60 -> 0.26 ms; it was
+// eight passes over V-word arrays, one thread writing all of a hub's
+// entries, and a check of one load in flight per thread.
+constexpr uint32_t kHeavyTile = 1024;
+
+__global__ void k_heavy_tiles(const uint32_t* row, uint32_t V, uint32_t ntiles, unsigned long long* sums,
                               uint32_t* bits, uint32_t* maxdeg) {
   const Warps W = warps_of(blockIdx.x, gridDim.x);
   const int lane = lane_id();
   uint32_t md = 0;
-  for (uint32_t base = W.gwarp * 32; base < V; base += W.nwarps * 32) {
-    const uint32_t v = base + lane;
-    const uint32_t d = v < V ? row[v + 1] - row[v] : 0u;
-    const bool hv = d > kHeavyDeg;
-    if (v < V) {
-      flag[v] = hv;
-      nch[v] = hv ? chunks_of(d) : 0u;
+  for (uint32_t t = W.gwarp; t < ntiles; t += W.nwarps) {
+    uint32_t nh = 0, nc = 0;
+#pragma unroll 4
+    for (uint32_t k = 0; k < kHeavyTile / 32; ++k) {
+      const uint32_t base = t * kHeavyTile + k * 32, v = base + lane;
+      const uint32_t d = v < V ? row[v + 1] - row[v] : 0u;
+      const unsigned m = __ballot_sync(kFull, d > kHeavyDeg);
+      if (lane == 0 && base < V) bits[base >> 5] = m;
+      nh += __popc(m);
+      nc += d > kHeavyDeg ? chunks_of(d) : 0u;
+      md = max(md, d);
     }
-    const unsigned m = __ballot_sync(kFull, hv);
-    if (lane == 0) bits[base >> 5] = m;
-    md = max(md, d);
+    nc = __reduce_add_sync(kFull, nc);
+    if (lane == 0) sums[t] = ((unsigned long long)nh << 32) | nc;
   }
   md = __reduce_max_sync(kFull, md);
   if (lane == 0 && md) atomicMax(maxdeg, md);
 }
 
-// Heavy vertex list and chunk entries {vertex, chunk, heavy index, chunks}.
-__global__ void k_heavy_fill(const uint32_t* row, uint32_t V, const uint32_t* flag,
-                             const uint32_t* hidx, const uint32_t* cbase, uint32_t* heavy_v,
-                             uint4* chunks) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    if (!flag[v]) continue;
-    const uint32_t h = hidx[v], n = chunks_of(row[v + 1] - row[v]), cb = cbase[v];
-    heavy_v[h] = v;
-    for (uint32_t j = 0; j < n; ++j) chunks[cb + j] = make_uint4(v, j, h, n);
+// One CTA: exclusive scan of the tiles' counts in place; *total gets the sum.
+__global__ void __launch_bounds__(kScanThreads) k_heavy_scan(unsigned long long* sums, uint32_t ntiles,
+                                                             unsigned long long* total) {
+  __shared__ unsigned long long wsum[kScanThreads / 32];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  unsigned long long carry = 0;
+  for (uint32_t b = 0; b < ntiles; b += kScanThreads) {
+    const uint32_t i = b + threadIdx.x;
+    const unsigned long long x = i < ntiles ? sums[i] : 0ull;
+    unsigned long long inc = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(kFull, inc, o);
+      if (lane >= o) inc += y;
+    }
+    __syncthreads();
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    unsigned long long before = carry, all = 0;
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+      if (w < warp) before += wsum[w];
+      all += wsum[w];
+    }
+    if (i < ntiles) sums[i] = before + inc - x;
+    carry += all;
+  }
+  if (threadIdx.x == 0) *total = carry;
+}
+
+// Heavy vertex list and chunk entries {vertex, chunk, heavy index, chunks}:
+// a CTA of eight warps per tile, an eighth of its vertices each (the first
+// tile of an R-MAT graph holds a thousand hubs of up to thousands of chunks;
+// one warp took 140 us over it).
+__global__ void __launch_bounds__(256) k_heavy_fill(const uint32_t* row, uint32_t V, uint32_t ntiles,
+                                                    const unsigned long long* sums, uint32_t* heavy_v,
+                                                    uint4* chunks) {
+  constexpr uint32_t kSteps = kHeavyTile / 256;  // 32-vertex steps per warp
+  __shared__ unsigned long long part[8];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const uint32_t first = t * kHeavyTile + warp * kSteps * 32;
+    uint32_t n[kSteps], nh = 0, nc = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kSteps; ++k) {
+      const uint32_t v = first + k * 32 + lane;
+      const uint32_t d = v < V ? row[v + 1] - row[v] : 0u;
+      n[k] = d > kHeavyDeg ? chunks_of(d) : 0u;
+      nh += __popc(__ballot_sync(kFull, n[k] != 0));
+      nc += n[k];
+    }
+    nc = __reduce_add_sync(kFull, nc);
+    __syncthreads();
+    if (lane == 0) part[warp] = ((unsigned long long)nh << 32) | nc;
+    __syncthreads();
+    unsigned long long at = sums[t];
+    for (int w = 0; w < warp; ++w) at += part[w];
+    uint32_t h = (uint32_t)(at >> 32), cb = (uint32_t)at;
+#pragma unroll
+    for (uint32_t k = 0; k < kSteps; ++k) {
+      const uint32_t base = first + k * 32;
+      for (unsigned m = __ballot_sync(kFull, n[k] != 0); m; m &= m - 1) {
+        const int o = __ffs(m) - 1;
+        const uint32_t nv = __shfl_sync(kFull, n[k], o);
+        if (lane == 0) heavy_v[h] = base + o;
+        for (uint32_t j = lane; j < nv; j += 32) chunks[cb + j] = make_uint4(base + o, j, h, nv);
+        ++h;
+        cb += nv;
+      }
+    }
   }
 }
 
@@ -356,82 +426,96 @@ void arc_split_drop(gdb_graph* g) {
   g->split_bound = 0;
 }
 
-// Heavy table of a derived CSR whose row array is on the device; `t0`,
-// `t1` (V + 1 words each) and `tmp` are scratch.
-static int heavy_table_device(gdb_ctx* c, gdb_graph* x, uint32_t* t0, uint32_t* t1, uint32_t* t2,
-                              uint32_t* t3, uint32_t* tmp, uint32_t* hs) {
-  const uint32_t V = x->V;
-  cudaStream_t st = c->stream;
-  const size_t nb = ((size_t)(V + 31) / 32 + 1) * 4;
-  GDB_CUDA(c, dev_alloc(c, (void**)&x->heavy_bits, nb));
-  GDB_CUDA(c, cudaMemsetAsync(x->heavy_bits, 0, nb, st));
-  GDB_CUDA(c, cudaMemsetAsync(hs, 0, 16, st));
-  const int grid = 8 * c->sm_count;  // every 256-thread CTA resident: the loops are latency-bound
-  k_heavy_marks<<<grid, 256, 0, st>>>(x->row, V, t0, t1, x->heavy_bits, hs + 2);
-  GDB_CUDA(c, cudaGetLastError());
-  GDB_CUDA(c, exclusive_scan(t0, V, t2, tmp, st));
-  GDB_CUDA(c, exclusive_scan(t1, V, t3, tmp, st));
-  GDB_CUDA(c, cudaMemcpyAsync(hs, t2 + V, 4, cudaMemcpyDeviceToDevice, st));
-  GDB_CUDA(c, cudaMemcpyAsync(hs + 1, t3 + V, 4, cudaMemcpyDeviceToDevice, st));
-  uint32_t* hh = (uint32_t*)pinned(c, 64);
-  if (!hh) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hh, hs, 12, cudaMemcpyDeviceToHost, st));
-  GDB_CUDA(c, cudaStreamSynchronize(st));
-  x->nheavy = hh[0];
-  x->nheavy_chunks = hh[1];
-  x->maxdeg = hh[2];
-  GDB_CUDA(c, dev_alloc(c, (void**)&x->heavy_v, std::max<size_t>(x->nheavy, 1) * 4));
-  GDB_CUDA(c, dev_alloc(c, (void**)&x->heavy_chunk, std::max<size_t>(x->nheavy_chunks, 1) * sizeof(uint4)));
-  k_heavy_fill<<<grid, 256, 0, st>>>(x->row, V, t0, t2, t3, x->heavy_v, x->heavy_chunk);
-  GDB_CUDA(c, cudaGetLastError());
-  return GDB_OK;
-}
-
 // One pass over a CSR's arrays: bit 0 when a row pointer decreases, bit 1
 // when a column names a vertex >= V -- a graph every kernel would read or
-// write out of bounds.
+// write out of bounds -- and bit 2 when the row pointers do not span the E
+// arcs (the columns are not read then).  The columns are a stream with
+// nothing behind it: 16-byte groups, four in flight per thread, and the few
+// words before and after them singly.
 __global__ void k_check_csr(const uint32_t* __restrict__ row, const uint32_t* __restrict__ col, uint32_t V,
                             uint64_t E, uint32_t* bad) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t b = 0;
+  uint32_t b = __ldg(&row[0]) != 0 || __ldg(&row[V]) != E ? 4u : 0u;
   for (uint64_t i = t0; i < V; i += stride) b |= __ldg(&row[i + 1]) < __ldg(&row[i]) ? 1u : 0u;
-  for (uint64_t e = t0; e < E; e += stride) b |= __ldg(&col[e]) >= V ? 2u : 0u;
+  if (!(b & 4u)) {
+    const uint64_t lead = ((16u - ((uintptr_t)col & 15u)) & 15u) / 4u, head = lead < E ? lead : E;
+    const uint64_t n4 = (E - head) / 4, tail = head + 4 * n4;
+    const uint4* c4 = reinterpret_cast<const uint4*>(col + head);
+    uint32_t top = 0;
+    if (t0 < head) top = __ldg(&col[t0]);
+    if (tail + t0 < E) top = max(top, __ldg(&col[tail + t0]));
+    for (uint64_t i = t0; i < n4; i += 4 * stride) {
+      uint4 q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = i + k * stride < n4 ? __ldg(&c4[i + k * stride]) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) top = max(max(top, max(q[k].x, q[k].y)), max(q[k].z, q[k].w));
+    }
+    if (top >= V) b |= 2u;
+  }
   b = __reduce_or_sync(0xffffffffu, b);
   if ((threadIdx.x & 31) == 0 && b) atomicOr(bad, b);
 }
 
-// The heavy table of a graph whose row array is on the device (every graph
-// the library creates): scratch of its own, one synchronisation for the
-// CSR check and one for the totals.  The check runs first: the table's
-// degrees come from the row array.
+// Heavy table of a CSR whose row array is on the device; with `check`, the
+// CSR check runs beside it and its bits come back with the totals (a bad
+// graph's totals are not used).  One synchronisation.
+static int heavy_table_device(gdb_ctx* c, gdb_graph* x, bool check, uint32_t* bad) {
+  const uint32_t V = x->V;
+  cudaStream_t st = c->stream;
+  const uint32_t ntiles = (V + kHeavyTile - 1) / kHeavyTile;
+  const size_t nb = ((size_t)(V + 31) / 32 + 1) * 4;
+  *bad = 0;
+  char* scratch = nullptr;  // {totals, largest degree, check bits}, tile counts
+  GDB_CUDA(c, cudaMallocAsync((void**)&scratch, 16 + (size_t)ntiles * 8, st));
+  unsigned long long *total = (unsigned long long*)scratch, *sums = total + 2;
+  uint32_t* word = (uint32_t*)scratch;
+  uint32_t* hh = (uint32_t*)pinned(c, 64);
+  cudaError_t e = hh ? dev_alloc(c, (void**)&x->heavy_bits, nb) : cudaErrorMemoryAllocation;
+  if (e == cudaSuccess) e = cudaMemsetAsync(x->heavy_bits, 0, nb, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(scratch, 0, 16, st);
+  const int grid = 8 * c->sm_count;  // every 256-thread CTA resident: the loops are latency-bound
+  if (e == cudaSuccess && check) {
+    k_check_csr<<<grid, 256, 0, st>>>(x->row, x->col, V, x->E, word + 3);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    k_heavy_tiles<<<grid, 256, 0, st>>>(x->row, V, ntiles, sums, x->heavy_bits, word + 2);
+    k_heavy_scan<<<1, kScanThreads, 0, st>>>(sums, ntiles, total);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hh, scratch, 16, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && !(*bad = hh[3])) {
+    x->nheavy_chunks = hh[0];
+    x->nheavy = hh[1];
+    x->maxdeg = hh[2];
+    e = dev_alloc(c, (void**)&x->heavy_v, std::max<size_t>(x->nheavy, 1) * 4);
+    if (e == cudaSuccess)
+      e = dev_alloc(c, (void**)&x->heavy_chunk, std::max<size_t>(x->nheavy_chunks, 1) * sizeof(uint4));
+    if (e == cudaSuccess && x->nheavy) {
+      k_heavy_fill<<<grid, 256, 0, st>>>(x->row, V, ntiles, sums, x->heavy_v, x->heavy_chunk);
+      e = cudaGetLastError();
+    }
+  }
+  cudaFreeAsync(scratch, st);
+  return e == cudaSuccess ? GDB_OK : set_cuda_error(c, e, "heavy table");
+}
+
+// The CSR check and the heavy table of a graph whose arrays are on the
+// device (every graph the library creates).
 int build_heavy_table(gdb_graph* g) {
   gdb_ctx* c = g->ctx;
-  const uint32_t V = g->V;
-  const size_t vw = (size_t)V + 1;
-  uint32_t* scratch = nullptr;
-  GDB_CUDA(c, cudaMallocAsync((void**)&scratch, (4 * vw + scan_tmp_words(V) + 8) * 4, c->stream));
-  uint32_t *t0 = scratch, *t1 = t0 + vw, *t2 = t1 + vw, *t3 = t2 + vw, *tmp = t3 + vw,
-           *hs = tmp + scan_tmp_words(V);
   uint32_t bad = 0;
-  cudaError_t ce = cudaMemsetAsync(hs + 7, 0, 4, c->stream);
-  if (ce == cudaSuccess) {
-    k_check_csr<<<4 * std::max(c->sm_count, 1), 256, 0, c->stream>>>(g->row, g->col, V, g->E, hs + 7);
-    ce = cudaGetLastError();
-  }
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&bad, hs + 7, 4, cudaMemcpyDeviceToHost, c->stream);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(c->stream);
-  if (ce != cudaSuccess || bad) {
-    cudaFreeAsync(scratch, c->stream);
-    cudaStreamSynchronize(c->stream);
-    if (ce != cudaSuccess) return set_cuda_error(c, ce, "CSR check");
-    return set_error(c, GDB_ERR_INVALID, (bad & 1) ? "row_ptr decreases" : "a column names a vertex >= V");
-  }
-  const int rc = heavy_table_device(c, g, t0, t1, t2, t3, tmp, hs);
-  cudaFreeAsync(scratch, c->stream);
+  const int rc = heavy_table_device(c, g, true, &bad);
   const cudaError_t e = cudaStreamSynchronize(c->stream);
   if (rc) return rc;
-  return e == cudaSuccess ? GDB_OK : set_cuda_error(c, e, "heavy table");
+  if (e != cudaSuccess) return set_cuda_error(c, e, "heavy table");
+  if (bad)
+    return set_error(c, GDB_ERR_INVALID, (bad & 4) ? "row_ptr[0] != 0 or row_ptr[V] != E"
+                                         : (bad & 1) ? "row_ptr decreases" : "a column names a vertex >= V");
+  return GDB_OK;
 }
 
 static gdb_graph* new_half(gdb_ctx* c, uint32_t V) {
@@ -450,13 +534,13 @@ int arc_split(gdb_ctx* c, gdb_graph* g, uint32_t bound) {
   gdb_graph* L = new_half(c, V);
   gdb_graph* H = new_half(c, V);
   gdb_graph* T = nullptr;  // transpose of H, built last
-  // scratch: four V + 1 word arrays, the scan's tile sums, totals, and
-  // four arrays over the heavy chunks (counts and their scans)
+  // scratch: two V + 1 word arrays, the scan's tile sums, and four arrays
+  // over the heavy chunks (counts and their scans)
   const size_t vw = (size_t)V + 1;
   const uint32_t nch = g->nheavy_chunks;
   const size_t cw = (size_t)nch + 1;
   uint32_t* scratch = nullptr;
-  const size_t words = 4 * vw + std::max(scan_tmp_words(V), scan_tmp_words(nch)) + 8 + 4 * cw;
+  const size_t words = 2 * vw + std::max(scan_tmp_words(V), scan_tmp_words(nch)) + 4 * cw;
   int rc = GDB_OK;
   auto fail = [&](int r) {
     if (scratch) cudaFreeAsync(scratch, st);
@@ -468,9 +552,9 @@ int arc_split(gdb_ctx* c, gdb_graph* g, uint32_t bound) {
   };
   cudaError_t e = cudaMallocAsync((void**)&scratch, words * 4, st);
   if (e != cudaSuccess) return fail(set_cuda_error(c, e, "arc split scratch"));
-  uint32_t *t0 = scratch, *t1 = t0 + vw, *t2 = t1 + vw, *t3 = t2 + vw, *tmp = t3 + vw,
-           *hs = tmp + std::max(scan_tmp_words(V), scan_tmp_words(nch)), *cl_c = hs + 8, *ch_c = cl_c + cw,
-           *pl_c = ch_c + cw, *ph_c = pl_c + cw;
+  uint32_t *t0 = scratch, *t1 = t0 + vw, *tmp = t1 + vw,
+           *cl_c = tmp + std::max(scan_tmp_words(V), scan_tmp_words(nch)), *ch_c = cl_c + cw, *pl_c = ch_c + cw,
+           *ph_c = pl_c + cw;
   e = dev_alloc(c, (void**)&L->row, vw * 4);
   if (e == cudaSuccess) e = dev_alloc(c, (void**)&H->row, vw * 4);
   if (e != cudaSuccess) return fail(set_cuda_error(c, e, "arc split rows"));
@@ -502,8 +586,9 @@ int arc_split(gdb_ctx* c, gdb_graph* g, uint32_t bound) {
   k_split_scatter<<<grid, 256, 0, st>>>(G, bound, L->row, H->row, pl_c, ph_c, L->col, L->w, H->col, H->w);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(set_cuda_error(c, e, "arc split scatter"));
-  if ((rc = heavy_table_device(c, L, t0, t1, t2, t3, tmp, hs))) return fail(rc);
-  if ((rc = heavy_table_device(c, H, t0, t1, t2, t3, tmp, hs))) return fail(rc);
+  uint32_t bad = 0;
+  if ((rc = heavy_table_device(c, L, false, &bad))) return fail(rc);
+  if ((rc = heavy_table_device(c, H, false, &bad))) return fail(rc);
   // the transpose of the heavy half: in-arcs with their weights, for the
   // pull form of a settle superstep -- a graph declared symmetric (with
   // symmetric weights) is its own transpose

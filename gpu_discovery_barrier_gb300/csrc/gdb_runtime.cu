@@ -515,11 +515,12 @@ int gdb_graph_create_device(gdb_ctx* c, uint32_t V, uint64_t E, const uint32_t* 
   *out = nullptr;
   int rc = graph_common(c, V, E);
   if (rc) return rc;
-  uint32_t ends[2] = {1, 0};
-  cudaError_t e = cudaMemcpy(&ends[0], d_row, 4, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(&ends[1], d_row + V, 4, cudaMemcpyDeviceToHost);
+  // a synchronous copy, which also waits for arrays still being written on
+  // the default stream; the check kernel looks at row_ptr[0]
+  uint32_t end = 0;
+  cudaError_t e = cudaMemcpy(&end, d_row + V, 4, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return set_cuda_error(c, e, "row_ptr read-back");
-  if (ends[0] != 0 || ends[1] != E) return set_error(c, GDB_ERR_INVALID, "row_ptr[0] != 0 or row_ptr[V] != E");
+  if (end != E) return set_error(c, GDB_ERR_INVALID, "row_ptr[0] != 0 or row_ptr[V] != E");
   gdb_graph* g = new gdb_graph();
   g->ctx = c;
   g->V = V;
