@@ -17,8 +17,9 @@
 //    count into every level-L+1 neighbour's (an FP32 L2 atomic, as the
 //    reference's float adds; FP64 ones cost 6 % more of the BC time); pull -- every unvisited vertex sums the path counts of its
 //    level-L neighbours and claims itself when the sum is positive.  A
-//    pull has no early exit (every parent counts), so it runs only when the
-//    unvisited vertices' arcs are fewer than the level's own;
+//    pull has no early exit (every parent counts), so it runs when the
+//    unvisited vertices' arcs are fewer than three times the level's own (a
+//    pushed arc ends in an atomic);
 //  * backward, level L (deepest first): levels below the level with the
 //    most arcs pull (1 + sigma[w]) / rho[w] from their level-L+1
 //    neighbours, levels above it push their own coefficient into their
@@ -45,14 +46,21 @@ namespace {
 
 using namespace gdb;
 
-// Per-vertex state.  st: x = level (int32, -1 = unreached), y = the
-// backward coefficient (1 + sigma) / rho (float bits), one 8-byte load for
-// the arcs of either pass; rho: the path count, float as the reference's
-// (pushes add into it with FP32 L2 atomics); sacc: FP64 accumulator of the
+// Per-vertex state.  st: x = level (int32, -1 = unreached), y = float bits:
+// the path count while the level lists grow (pushes add into it with FP32 L2
+// atomics, float as the reference's), then, from the peak level down, the
+// backward coefficient (1 + sigma) / rho -- one 8-byte load for the arcs of
+// either pass (counts in an array of their own made a pulled arc two L2
+// sectors, and pulls are bound by those).  Coefficients of levels above the
+// peak are pushed, never read, and not stored, so a count stays readable for
+// every chunk of a heavy vertex there.  sacc: FP64 accumulator of the
 // backward sum of pushed levels.
+// The pulls' and the backward pushes' loads of st are ordinary ones, through
+// L1: what they look for was final at the last barrier, whose acquire drops
+// older lines, and a stale level of a vertex being claimed is not the one
+// looked for either.
 struct BcWs {
   uint2* st;
-  float* rho;
   double* sacc;
   float* bc;
   uint32_t* order;               // light vertices, level segments
@@ -151,11 +159,15 @@ __device__ __forceinline__ int32_t level_of(const BcWs& ws, uint32_t v) {
   return (int32_t)__ldcg(reinterpret_cast<const uint32_t*>(&ws.st[v]));
 }
 __device__ __forceinline__ float rho_of(const BcWs& ws, uint32_t v) {
-  return __ldcg(&ws.rho[v]);
+  return __uint_as_float(__ldcg(&ws.st[v].y));
 }
 __device__ __forceinline__ void set_coef(const BcWs& ws, uint32_t v, float c) {
   reinterpret_cast<uint32_t*>(&ws.st[v])[1] = __float_as_uint(c);
 }
+// A pulled arc costs a third of a pushed one, which ends in an atomic (R-MAT-22,
+// 16 sources, a level pulled when mu + V < kBcPull x mf: 1 17.7 ms, 2 16.9, 3 and
+// 4 15.2, 6 15.4).
+constexpr unsigned long long kBcPull = 3;
 constexpr uint2 kUnreached = {0xFFFFFFFFu, 0u};
 // an empty sum: sums start at -0.0, and -0.0 + x = x for every x >= +0.0
 __device__ __forceinline__ bool no_terms(double s) { return s == 0.0 && signbit(s); }
@@ -209,7 +221,6 @@ __device__ __forceinline__ uint32_t bc_degree(const GraphView& G, uint32_t v) {
 __device__ __forceinline__ void bc_init(const GraphView& G, const Warps& W, const BcWs& ws, bool leader) {
   for (uint32_t v = W.gthread; v < G.V; v += W.nthreads) {
     ws.st[v] = kUnreached;
-    ws.rho[v] = 0.f;
     ws.sacc[v] = -0.0;
     ws.bc[v] = 0.f;
   }
@@ -239,8 +250,7 @@ __device__ __forceinline__ void bc_seed(const GraphView& G, const BcWs& ws, uint
     return;
   }
   if (leader) {
-    ws.st[src] = make_uint2(0u, 0u);
-    ws.rho[src] = 1.f;
+    ws.st[src] = make_uint2(0u, __float_as_uint(1.f));
     ws.lev_arcs[0] = degree(src);
     ws.lev_arcs[1] = 0;
     const int nx = (t + 1) % 3;
@@ -294,9 +304,9 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
   // direction of L -> L+1, from the same counters in every CTA: a push
   // walks the level's mf arcs, a pull (no early exit: every parent
   // counts) the arcs of every unvisited vertex plus one look at each
-  // vertex's level -- the cheaper one runs
+  // vertex's level -- the cheaper one runs (kBcPull)
   const unsigned long long mu = G.E > vis_arcs ? G.E - vis_arcs : 0ull;
-  const bool pull = mu + G.V < mf;
+  const bool pull = mu + G.V < kBcPull * mf;
   const uint32_t nlbase = lbase + nl, nhcbase = hcbase + nch, nhvbase = hvbase + nhv;
   Frontier out{ws.order + nlbase, ws.hc + nhcbase, &ws.lcnt[nx], &ws.hcnt[nx], G.V - nlbase,
                ws.hc_cap - nhcbase, ws.overflow, G.nheavy - nhvbase, ws.hleft + nhvbase,
@@ -334,7 +344,7 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
         const bool claimed = du[j] == -1 && old[j] == -1;
         const bool add = du[j] == Li + 1 || claimed || (du[j] == -1 && old[j] == Li + 1);
         if (claimed) next_arcs += r1[j] - r0[j];
-        if (add) atomicAdd(&ws.rho[u[j]], rv[j]);
+        if (add) atomicAdd(reinterpret_cast<float*>(&ws.st[u[j]].y), rv[j]);
         frontier_push_staged(G, out, qs, claimed, u[j]);
       }
     };
@@ -364,39 +374,76 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
   } else {
     // pull: every unvisited vertex sums the path counts of its level-L
     // neighbours (all of them) and claims itself when there are any
-    for (uint32_t g = W.gwarp; g * 32 < G.V; g += W.nwarps) {
+    for_groups((G.V + 31) / 32, W, &ws.cursor[cur], 64, [&](uint32_t g) {
       const uint32_t u = g * 32 + lane;
-      const bool unv = u < G.V && level_of(ws, u) == -1;
+      const bool unv = u < G.V && !is_heavy(G, u) && level_of(ws, u) == -1;
       my[lane] = 0.0;
       __syncwarp();
-      // four steps at once; a neighbour's path count is loaded with its
-      // level (and used only when the level is L)
+      // four steps at once
       group_arcs4(G, unv, u, [&](const bool* valid, const int* owner, const uint32_t* arc) {
         uint32_t w[4];
-        int32_t lw[4];
-        float rw[4];
+        uint2 sw[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           w[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
           arcs += valid[j];
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          lw[j] = valid[j] ? level_of(ws, w[j]) : -2;
-          rw[j] = valid[j] ? rho_of(ws, w[j]) : 0.f;
-        }
+        for (int j = 0; j < 4; ++j) sw[j] = valid[j] ? ws.st[w[j]] : kUnreached;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) segment_add(my, owner[j], lw[j] == Li ? rw[j] : -0.f);  // -0: no term
+        for (int j = 0; j < 4; ++j)  // -0: no term
+          segment_add(my, owner[j], (int32_t)sw[j].x == Li ? __uint_as_float(sw[j].y) : -0.f);
       });
       __syncwarp();
       const double sum = my[lane];
       const bool claimed = unv && sum > 0.0;
       if (claimed) {
-        ws.st[u].x = (uint32_t)(Li + 1);  // only this lane writes u
-        ws.rho[u] = (float)sum;
+        ws.st[u] = make_uint2((uint32_t)(Li + 1), __float_as_uint((float)sum));  // only this lane writes u
         next_arcs += degree(u);
       }
       frontier_push_staged(G, out, qs, claimed, u);
+    });
+    // the unvisited heavy vertices chunk by chunk (a hub left to one warp
+    // held the level up for hundreds of microseconds): the first chunk with
+    // a parent claims the vertex, each adds its FP32 sum as a push would
+    while (nhvbase < G.nheavy) {  // some left
+      const uint32_t base = warp_grab(&ws.hcursor[cur]) * 32;
+      if (base >= G.nheavy_chunks) break;
+      const uint4 ent = base + lane < G.nheavy_chunks ? __ldg(&G.heavy_chunk[base + lane]) : make_uint4(0, 0, 0, 0);
+      // L + 1: claimed by another chunk in this superstep
+      const int32_t lu = ent.w ? level_of(ws, ent.x) : -2;
+      const bool open = lu == -1 || lu == Li + 1;
+      uint32_t rb = 0, re = 0;
+      if (open) {
+        rb = __ldg(&G.row[ent.x]) + ent.y * kChunk;
+        re = min(__ldg(&G.row[ent.x + 1]), rb + kChunk);
+      }
+      for (unsigned todo = __ballot_sync(kFull, open); todo; todo &= todo - 1) {
+        const int o = __ffs(todo) - 1;
+        const uint32_t u = __shfl_sync(kFull, ent.x, o);
+        bool valid[4];
+        uint32_t arc[4], w[4];
+        uint2 sw[4];
+        chunk_steps(__shfl_sync(kFull, rb, o), __shfl_sync(kFull, re, o), valid, arc);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          w[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
+          arcs += valid[j];
+        }
+        float part = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sw[j] = valid[j] ? ws.st[w[j]] : kUnreached;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part += (int32_t)sw[j].x == Li ? __uint_as_float(sw[j].y) : 0.f;
+        part = warp_sum_f32(part);
+        bool claimed = false;
+        if (lane == 0 && part > 0.f) {
+          claimed = atomicCAS(reinterpret_cast<int*>(&ws.st[u].x), -1, Li + 1) == -1;
+          atomicAdd(reinterpret_cast<float*>(&ws.st[u].y), part);
+          if (claimed) next_arcs += degree(u);
+        }
+        if (__any_sync(kFull, claimed)) frontier_push_staged(G, out, qs, claimed, u);
+      }
     }
     if (leader) reached_arcs += mf;
   }
@@ -433,7 +480,7 @@ __device__ __forceinline__ void bc_backward(const GraphView& G, const Warps& W, 
   // overflowed (coefficient 0) still gives inf x 0 = NaN, as there
   auto finalize = [&](uint32_t v, float rv, double sum) {
     const float sg = no_terms(sum) ? 0.f : (float)((double)rv * sum);
-    set_coef(ws, v, (1.0f + sg) / rv);
+    if ((uint32_t)Lb <= peak) set_coef(ws, v, (1.0f + sg) / rv);
     if (v != src) ws.bc[v] += sg;
     return (1.0f + sg) / rv;
   };
@@ -450,7 +497,7 @@ __device__ __forceinline__ void bc_backward(const GraphView& G, const Warps& W, 
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)  // level and coefficient
-        su[j] = valid[j] ? __ldcg(&ws.st[c[j]]) : make_uint2(0xFFFFFFFFu, 0u);
+        su[j] = valid[j] ? ws.st[c[j]] : kUnreached;
 #pragma unroll
       for (int j = 0; j < 4; ++j) a[j] = (int32_t)su[j].x == Lb + 1 ? __uint_as_float(su[j].y) : -0.f;
     };
@@ -507,7 +554,7 @@ __device__ __forceinline__ void bc_backward(const GraphView& G, const Warps& W, 
         arcs += valid[j];
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) lu[j] = valid[j] ? level_of(ws, u[j]) : -2;
+      for (int j = 0; j < 4; ++j) lu[j] = valid[j] ? (int32_t)ws.st[u[j]].x : -2;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (lu[j] == Lb - 1) atomicAdd(&ws.sacc[u[j]], (double)cf[j]);
@@ -552,7 +599,6 @@ __device__ __forceinline__ void bc_reset(const GraphView& G, const Warps& W, con
   // -- reset the reached vertices for the next source
   auto reset = [&](uint32_t v) {
     ws.st[v] = kUnreached;
-    ws.rho[v] = 0.f;
     ws.sacc[v] = -0.0;
   };
   for (uint32_t k = W.gthread; k < total_l; k += W.nthreads) reset(ws.order[k]);
@@ -753,8 +799,7 @@ static size_t bc_layout(const gdb_graph* g, char* base, float* d_bc, const uint3
   const uint32_t ccap = std::max<uint32_t>(g->nheavy_chunks, 1);
   const uint32_t maxlev = V + 2;
   Bump b;
-  const size_t o_st = b.take((size_t)V * 8), o_rho = b.take((size_t)V * 8),
-               o_sacc = b.take((size_t)V * 8);
+  const size_t o_st = b.take((size_t)V * 8), o_sacc = b.take((size_t)V * 8);
   const size_t o_ord = b.take((size_t)V * 4);
   const size_t o_hc = b.take((size_t)ccap * 16), o_hacc = b.take((size_t)hcap * 8),
                o_hleft = b.take((size_t)hcap * 4);
@@ -764,7 +809,6 @@ static size_t bc_layout(const gdb_graph* g, char* base, float* d_bc, const uint3
   const size_t o_cnt = b.take(512);
   if (!base) return b.off;
   ws->st = (uint2*)(base + o_st);
-  ws->rho = (float*)(base + o_rho);
   ws->sacc = (double*)(base + o_sacc);
   ws->bc = d_bc;
   ws->order = (uint32_t*)(base + o_ord);
@@ -814,8 +858,8 @@ int gdbi::bc_enqueue(gdb_ctx* c, gdb_graph* g, void* wsbase, const uint32_t* d_s
 // Several sources: contiguous groups of them on concurrent lanes, each
 // lane summing into its own array, then one pass adds the lanes' arrays.
 // Four lanes: BC's launches are longer and fuller than BFS's and SSSP's
-// (R-MAT-22, 16 sources: 16.7 ms on two lanes, 16.2 on four, 18.2 on
-// eight, 27.3 on sixteen; on one launch, an earlier build took 20.9 ms).
+// (R-MAT-22, 16 sources: 16.6 ms on two lanes, 15.2 on four, 16.9 on six,
+// 15.7 on eight, in one call; 27.3 on sixteen in an earlier build).
 constexpr uint32_t kBcLanes = 4;
 
 static int bc_lanes(gdb_ctx* c, gdb_graph* g, const uint32_t* d_sources, uint32_t nsrc, float* d_bc) {

@@ -36,8 +36,8 @@ constexpr uint32_t kGrab = 4;
 // warp, and the superstep waits for the densest (four against always kGrab:
 // MST on 5,000 / 60,000 / 400,003 / 1,500,000 vertices 465 -> 316, 571 -> 401,
 // 941 -> 794, 1,571 -> 1,499 us; at 4 M vertices nothing changes)
-__device__ __forceinline__ uint32_t grab_of(uint32_t ngroups) {
-  const uint32_t per = ngroups / (4u * (gridDim.x * (blockDim.x >> 5)));
+__device__ __forceinline__ uint32_t grab_of(uint32_t ngroups, uint32_t grabs = 4) {
+  const uint32_t per = ngroups / (grabs * (gridDim.x * (blockDim.x >> 5)));
   return per < 1u ? 1u : per < kGrab ? per : kGrab;
 }
 // warps per CTA of the graph kernels (launch bounds of 512 threads)
@@ -517,6 +517,25 @@ __device__ __forceinline__ void visit_frontier4(const GraphView& G, const Warps&
   }
 }
 
+// The 32-vertex groups [0, ngroups) over the grid's warps.  From eight groups
+// per warp on they come from the cursor, in fixed strides only below: an
+// R-MAT vertex's degree follows the zero bits of its id, so the warps of one
+// residue class got the dense groups throughout (BC's pull of the 4 M
+// unvisited vertices of R-MAT-22: warps busy 188 us on average, the last 570).
+// grabs: how many a warp should get of its groups' share.  For sweeps that
+// walk whole lists: BFS's pull, which stops at the first parent, and SSSP's
+// settle lost by it (3,000,001 vertices, one source: 0.31 -> 0.38 and 1.63 ->
+// 1.68 ms).
+template <class Fn>
+__device__ __forceinline__ void for_groups(uint32_t ngroups, const Warps& W, uint32_t* cursor, uint32_t grabs,
+                                           Fn&& fn) {
+  const bool fixed = ngroups < 8u * W.nwarps;
+  const uint32_t grab = fixed ? 1u : grab_of(ngroups, grabs);
+  WorkTaker it((ngroups + grab - 1) / grab, W, cursor);
+  for (uint32_t i = it.take(); i < it.n; i = fixed ? i + W.nwarps : it.take())
+    for (uint32_t g = i * grab; g < min((i + 1) * grab, ngroups); ++g) fn(g);
+}
+
 // Sweep the light vertices of [0, V) in warp groups of 32 consecutive ids.
 // begin(v, in_range) -> bool active: per-lane setup (v is light and < V
 // when in_range); edge(valid, owner_lane, arc) per 32-arc step;
@@ -656,14 +675,17 @@ __device__ __forceinline__ void cta_or(bool p, uint32_t* word, uint32_t bit) {
 // a slot that starts at -0.0 still reads -0.0 when nothing was added.
 __device__ __forceinline__ void segment_add(double* slot, int owner, float x) {
   const int lane = lane_id();
+  const int prev = __shfl_up_sync(kFull, owner, 1);
+  const bool head = lane == 0 || prev != owner;
+  // lanes that follow in this one's segment
+  const unsigned next = __ballot_sync(kFull, head) & ~(lanemask_lt() | (1u << lane));
+  const int rest = (next ? __ffs(next) - 1 : 32) - 1 - lane;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const float y = __shfl_down_sync(kFull, x, o);
-    const int ow = __shfl_down_sync(kFull, owner, o);
-    if (lane + o < 32 && ow == owner) x += y;
+    if (o <= rest) x += y;
   }
-  const int prev = __shfl_up_sync(kFull, owner, 1);
-  if ((lane == 0 || prev != owner) && __float_as_uint(x) != 0x80000000u) slot[owner] += (double)x;
+  if (head && __float_as_uint(x) != 0x80000000u) slot[owner] += (double)x;
 }
 
 __device__ __forceinline__ float warp_sum_f32(float x) {
