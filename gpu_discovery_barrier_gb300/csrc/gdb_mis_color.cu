@@ -374,13 +374,12 @@ __global__ void __launch_bounds__(512, 3) k_mis_rl_step(GraphView G, MisWs ws, S
 struct ColorWs {
   int32_t* color;
   uint32_t* cnt;       // neighbours still to be coloured before this vertex
-  uint32_t* wcol;      // from row[v]: the wcnt[v] neighbours that wait for v (the count pass)
-  uint32_t* wcnt;
+  uint32_t* wcol;      // from row[v]: the neighbours that wait for v (the count pass)
+  uint2* run;          // v's run of them in wcol: {row[v], how many}
   const float* prio;
   uint2* q[2];                 // light vertices as their arc ranges {begin, end}
-  uint4* hc[2];                // heavy chunks as {vertex, first arc, end arc, chunk}
-  uint32_t* qcount;            // [3]
-  unsigned long long* hcount;  // [3]
+  uint2* hc[2];                // heavy chunks, likewise
+  unsigned long long* count;   // [3]: (chunks << 32) | light entries
   uint32_t* cursor;            // [3]
   uint32_t* hcursor;           // [3]
   int* overflow;
@@ -397,87 +396,102 @@ struct ColorWs {
 // kHeavyDeg neighbours wait for it.
 
 // The colouring's frontier entries carry arc ranges, so a round's consumer
-// needs no row load: the producer loads the rows of every vertex it counts
-// down, in flight with the count-down itself.  Light entries are staged per
-// warp in shared memory and leave 32 at a time; a heavy vertex's chunks are
-// reserved with one packed atomic per warp step.
-struct RangeStage {
-  uint2* buf;    // this warp's 64 slots
-  uint2* q;
-  uint32_t* count;
-  uint32_t cap;
-  int* overflow;
-  uint32_t n = 0;
-  __device__ __forceinline__ void out(uint2 x, uint32_t m) {
-    const int lane = lane_id();
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(count, m);
-    base = __shfl_sync(kFull, base, 0);
-    if ((uint32_t)lane < m) {
-      if (base + lane < cap) q[base + lane] = x;
-      else atomicExch(overflow, 1);
-    }
-  }
-  __device__ __forceinline__ void add(bool want, uint2 x) {
-    const unsigned m = __ballot_sync(kFull, want);
-    if (!m) return;
-    const int lane = lane_id();
-    if (want) buf[n + __popc(m & lanemask_lt())] = x;
-    n += __popc(m);
-    if (n >= 32) {
-      __syncwarp();
-      const uint2 y = buf[lane];
-      const uint32_t r = n - 32;
-      const uint2 z = (uint32_t)lane < r ? buf[32 + lane] : make_uint2(0u, 0u);
-      __syncwarp();
-      if ((uint32_t)lane < r) buf[lane] = z;
-      __syncwarp();
-      out(y, 32);
-      n = r;
-    }
-  }
-  __device__ __forceinline__ void flush() {
-    __syncwarp();
-    if (n) out((uint32_t)lane_id() < n ? buf[lane_id()] : make_uint2(0u, 0u), n);
-    n = 0;
-  }
-};
+// needs no row load: the producer loads the run of every vertex it counts
+// down, in flight with the count-down itself.
+//
+// What bounds it: a round is one chain of dependent round trips (counts and
+// entry, packed arcs, count-downs, reservation, entry stores, barrier), and a
+// power-law graph has thousands of rounds of a few hundred entries and some
+// 20,000 arcs.  R-MAT-22 (2,833 rounds): 20.0 -> 13.9 ms, of which the count
+// pass takes 1.1 and a round 4.5 us (barrier 1.3).  It came from the
+// predicated batch below (20.2 -> 15.8 with nothing else changed), from one
+// reservation for a batch's light entries and chunks instead of up to five in
+// turn, and from {row, count} runs read as one word pair (15.8 -> 13.9).
+// Measured and left out: fetching the runs' lines to L2 ahead (14.7), keeping
+// entries in the CTA that made them (14.8 light only, 19.4 with chunks: a warp
+// then has two entries in turn), starting on the entries before the counts are
+// known (14.5), writing the colours one batch later (14.1).
 
-// Push the lanes' ready vertices u with arc ranges [rb, re): light ones
-// (degree <= kHeavyDeg) staged, heavy ones as chunk entries.
-__device__ __forceinline__ void push_ranges(const ColorWs& ws, RangeStage& st, uint4* hc,
-                                            unsigned long long* hcount, bool ready, bool heavy,
-                                            uint32_t u, uint32_t rb, uint32_t re) {
-  st.add(ready && !heavy && re > rb, make_uint2(rb, re));
-  const bool hv = ready && heavy;
-  const unsigned hm = __ballot_sync(kFull, hv);
-  if (!hm) return;
+// Loads and count-downs under a predicate, as single instructions.  Written
+// as conditional expressions they became branches, and lanes that had parted
+// there went through the batch one group after the other, each with its own
+// round trips.
+__device__ __forceinline__ uint32_t ld_cg_if(bool p, const uint32_t* a) {
+  uint32_t x;
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; mov.u32 %0, 0; @p ld.global.cg.u32 %0, [%1]; }"
+               : "=r"(x) : "l"(a), "r"((uint32_t)p) : "memory");
+  return x;
+}
+__device__ __forceinline__ uint2 ld_cg_if(bool p, const uint2* a) {
+  uint2 x;
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %3, 0; mov.u32 %0, 0; mov.u32 %1, 0;\n"
+               " @p ld.global.cg.v2.u32 {%0, %1}, [%2]; }"
+               : "=r"(x.x), "=r"(x.y) : "l"(a), "r"((uint32_t)p) : "memory");
+  return x;
+}
+// *a - 1 under p, returning what it was (0 without p)
+__device__ __forceinline__ uint32_t count_down_if(bool p, uint32_t* a) {
+  uint32_t x;
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; mov.u32 %0, 0;\n"
+               " @p atom.global.add.u32 %0, [%1], -1; }"
+               : "=r"(x) : "l"(a), "r"((uint32_t)p) : "memory");
+  return x;
+}
+
+// Push the lanes' ready vertices of N steps, with their runs: a light one
+// (at most kHeavyDeg wait for it) as one entry, a heavy one as chunks.  One
+// reservation for both lists and all steps.
+template <int N>
+__device__ __forceinline__ void push_runs(const ColorWs& ws, uint2* q, uint2* hc, unsigned long long* count,
+                                          const bool (&ready)[N], const uint2 (&run)[N]) {
   const int lane = lane_id();
-  const uint32_t nch = hv ? chunks_of(re - rb) : 0u;
-  uint32_t inc = nch;
+  unsigned lm[N], hany = 0;
+  uint32_t nl = 0, nch = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(kFull, inc, o);
-    if (lane >= o) inc += t;
+  for (int j = 0; j < N; ++j) {
+    lm[j] = __ballot_sync(kFull, ready[j] && run[j].y - 1u < kHeavyDeg);
+    nl += __popc(lm[j]);
+    if (ready[j] && run[j].y > kHeavyDeg) nch += chunks_of(run[j].y);
   }
-  const uint32_t total = __shfl_sync(kFull, inc, 31);
-  const int leader = __ffs(hm) - 1;
-  unsigned long long old = 0;
-  if (lane == leader) old = atomicAdd(hcount, ((unsigned long long)__popc(hm) << 32) | total);
-  old = __shfl_sync(kFull, old, leader);
-  const uint32_t cbase = (uint32_t)old;
-  if (cbase + total > ws.hcap) {
-    if (lane == leader) atomicExch(ws.overflow, 1);
+  hany = __ballot_sync(kFull, nch);
+  uint32_t inc = nch;
+  if (hany) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, inc, o);
+      if (lane >= o) inc += t;
+    }
+  } else if (nl == 0) {
     return;
   }
-  const uint32_t first = cbase + inc - nch;
-  for (unsigned m = hm; m; m &= m - 1) {
-    const int l = __ffs(m) - 1;
-    const uint32_t v = __shfl_sync(kFull, u, l), n = __shfl_sync(kFull, nch, l);
-    const uint32_t f = __shfl_sync(kFull, first, l), b0 = __shfl_sync(kFull, rb, l),
-                   e0 = __shfl_sync(kFull, re, l);
-    for (uint32_t j = lane; j < n; j += 32)
-      hc[f + j] = make_uint4(v, b0 + j * kChunk, min(e0, b0 + (j + 1) * kChunk), j);
+  const uint32_t total = __shfl_sync(kFull, inc, 31);
+  unsigned long long at = 0;
+  if (lane == 0) at = atomicAdd(count, ((unsigned long long)total << 32) | nl);
+  at = __shfl_sync(kFull, at, 0);
+  uint32_t lbase = (uint32_t)at;
+  if (lbase + nl > ws.qcap || (uint32_t)(at >> 32) + total > ws.hcap) {
+    if (lane == 0) atomicExch(ws.overflow, 1);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if ((lm[j] >> lane) & 1u)
+      q[lbase + __popc(lm[j] & lanemask_lt())] = make_uint2(run[j].x, run[j].x + run[j].y);
+    lbase += __popc(lm[j]);
+  }
+  if (!hany) return;
+  uint32_t first = (uint32_t)(at >> 32) + inc - nch;  // of this lane's next heavy vertex
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const bool hv = ready[j] && run[j].y > kHeavyDeg;
+    for (unsigned m = __ballot_sync(kFull, hv); m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const uint32_t f = __shfl_sync(kFull, first, l);
+      const uint32_t b0 = __shfl_sync(kFull, run[j].x, l), n0 = __shfl_sync(kFull, run[j].y, l);
+      for (uint32_t k = lane; k < chunks_of(n0); k += 32)
+        hc[f + k] = make_uint2(b0 + k * kChunk, min(b0 + n0, b0 + (k + 1) * kChunk));
+    }
+    if (hv) first += chunks_of(run[j].y);
   }
 }
 
@@ -485,7 +499,10 @@ __device__ __forceinline__ void push_ranges(const ColorWs& ws, RangeStage& st, u
 __device__ __forceinline__ void color_init(const GraphView& G, const Warps& W, const ColorWs& ws) {
   for (uint32_t v = W.gthread; v < G.V; v += W.nthreads) {
     ws.color[v] = -1;
-    if (is_heavy(G, v)) ws.cnt[v] = ws.wcnt[v] = 0;
+    if (is_heavy(G, v)) {
+      ws.cnt[v] = 0;
+      ws.run[v] = make_uint2(__ldg(&G.row[v]), 0u);
+    }
   }
 }
 
@@ -539,7 +556,7 @@ __device__ __forceinline__ void color_count(const GraphView& G, const ColorWs& w
         [&](uint32_t v, bool) {
           if (v < G.V && !is_heavy(G, v)) {
             ws.cnt[v] = my[lane];
-            ws.wcnt[v] = wmy[lane];
+            ws.run[v] = make_uint2(rv_lane, wmy[lane]);
           }
         });
     sweep_heavy(G, &ws.hcursor[0], [&](uint32_t v, uint32_t, uint32_t, uint32_t b, uint32_t e) {
@@ -574,7 +591,7 @@ __device__ __forceinline__ void color_count(const GraphView& G, const ColorWs& w
       if (lane == 0 && n) atomicAdd(&ws.cnt[v], n);
       // the chunk's waiting neighbours: one reservation in v's packed run
       uint32_t at = 0;
-      if (lane == 0 && nw) at = atomicAdd(&ws.wcnt[v], nw);
+      if (lane == 0 && nw) at = atomicAdd(&ws.run[v].y, nw);
       at = rv + __shfl_sync(kFull, at, 0);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -587,32 +604,34 @@ __device__ __forceinline__ void color_count(const GraphView& G, const ColorWs& w
 
 // Superstep 2: vertices that wait for nobody take colour 1 (queue slot 1).
 __device__ __forceinline__ void color_first(const GraphView& G, const Warps& W, const ColorWs& ws, bool leader,
-                                            uint2 (*rstage)[64], unsigned long long& coloured) {
+                                            unsigned long long& coloured) {
   const int lane = lane_id();
-  {
-    RangeStage qs{rstage[threadIdx.x >> 5], pick(ws.q, 1), &ws.qcount[1], ws.qcap, ws.overflow};
-    for (uint32_t g = W.gwarp; g * 32 < G.V; g += W.nwarps) {
-      const uint32_t v = g * 32 + lane;
-      const bool first = v < G.V && ld_cg(&ws.cnt[v]) == 0;
-      uint32_t rb = 0, wn = 0;
-      if (first) {
-        ws.color[v] = 1;
-        ++coloured;
-        rb = __ldg(&G.row[v]);
-        wn = ld_cg(&ws.wcnt[v]);
-      }
-      push_ranges(ws, qs, pick(ws.hc, 1), &ws.hcount[1], first, wn > kHeavyDeg, v, rb, rb + wn);
+  for (uint32_t g = W.gwarp; g * 128 < G.V; g += W.nwarps) {
+    bool first[4];
+    uint32_t v[4];
+    uint2 run[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[j] = g * 128 + 32 * j + lane;
+      first[j] = v[j] < G.V && ld_cg(&ws.cnt[v[j]]) == 0;
+      run[j] = v[j] < G.V ? __ldcg(&ws.run[v[j]]) : make_uint2(0u, 0u);
     }
-    qs.flush();
-    if (leader) ws.cursor[2] = ws.hcursor[2] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (first[j]) {
+        ws.color[v[j]] = 1;
+        ++coloured;
+      }
+    }
+    push_runs<4>(ws, pick(ws.q, 1), pick(ws.hc, 1), &ws.count[1], first, run);
   }
+  if (leader) ws.cursor[2] = ws.hcursor[2] = 0;
 }
 
 // Round r: the vertices coloured in round r (queue slot r % 3) count down
 // the neighbours waiting for them; false when the round has no entries.
 __device__ __forceinline__ bool color_round(const GraphView& G, const Warps& W, const ColorWs& ws, uint32_t r,
-                                            bool leader, uint2 (*rstage)[64], unsigned long long& arcs,
-                                            unsigned long long& coloured) {
+                                            bool leader, unsigned long long& arcs, unsigned long long& coloured) {
   const int lane = lane_id();
   const int cur = r % 3, nxt = (r + 1) % 3, old = (r + 2) % 3;
   // Light groups go to the warps in spread order (warp 0 of every CTA,
@@ -625,27 +644,21 @@ __device__ __forceinline__ bool color_round(const GraphView& G, const Warps& W, 
   // (entries past the counts are never used).
   const uint32_t ls = W.spread, hs = W.nwarps - 1 - W.spread;
   const uint2* q = pick(ws.q, r);
-  const uint4* hc = pick(ws.hc, r);
+  const uint2* hc = pick(ws.hc, r);
   uint2 spec = make_uint2(0u, 0u);
   if (lane == 0 && ls < ws.qcap) spec = __ldcg(&q[ls]);
-  const uint4 hspec = hs < ws.hcap ? ld_cg(&hc[hs]) : make_uint4(0u, 0u, 0u, 0u);
-  const unsigned long long* sc = cta_words<2>([&](unsigned long long* w) {
-    w[0] = ld_cg(&ws.qcount[cur]);
-    w[1] = __ldcg(&ws.hcount[cur]);
-  });
-  const uint32_t n = (uint32_t)sc[0];
-  const unsigned long long hp = sc[1];
-  if (n == 0 && hp == 0) return false;
+  const uint2 hspec = hs < ws.hcap ? __ldcg(&hc[hs]) : make_uint2(0u, 0u);
+  const unsigned long long both =
+      *cta_words<1>([&](unsigned long long* w) { w[0] = __ldcg(&ws.count[cur]); });
+  const uint32_t n = (uint32_t)both, nch = (uint32_t)(both >> 32);
+  if (both == 0) return false;
   if (leader) {
-    ws.qcount[old] = 0;
-    ws.hcount[old] = 0;
+    ws.count[old] = 0;
     ws.cursor[old] = 0;
     ws.hcursor[old] = 0;
   }
-  RangeStage qs{rstage[threadIdx.x >> 5], pick(ws.q, r + 1), &ws.qcount[nxt], ws.qcap,
-                ws.overflow};
-  uint4* hc_out = pick(ws.hc, r + 1);
-  unsigned long long* hcount_out = &ws.hcount[nxt];
+  uint2* q_out = pick(ws.q, r + 1);
+  uint2* hc_out = pick(ws.hc, r + 1);
   const int32_t next_color = (int32_t)r + 1;
   // up to four 32-arc steps at once: their neighbour loads and
   // count-downs are all in flight together (a round is a chain of
@@ -655,27 +668,29 @@ __device__ __forceinline__ bool color_round(const GraphView& G, const Warps& W, 
     uint32_t u[4];
 #pragma unroll
     for (int s4 = 0; s4 < 4; ++s4) {
-      u[s4] = valid[s4] ? __ldcg(&ws.wcol[arc[s4]]) : 0u;
+      u[s4] = ld_cg_if(valid[s4], &ws.wcol[arc[s4]]);
       arcs += valid[s4];
     }
-    uint32_t old4[4], rb[4], wn[4];
+    __syncwarp();
+    uint32_t old4[4];
+    uint2 run[4];
 #pragma unroll
     for (int s4 = 0; s4 < 4; ++s4) {
-      old4[s4] = valid[s4] ? atomicSub(&ws.cnt[u[s4]], 1u) : 0u;
+      old4[s4] = count_down_if(valid[s4], &ws.cnt[u[s4]]);
       // the packed run of a vertex this count-down may complete, loaded
       // with it
-      rb[s4] = valid[s4] ? __ldg(&G.row[u[s4]]) : 0u;
-      wn[s4] = valid[s4] ? ld_cg(&ws.wcnt[u[s4]]) : 0u;
+      run[s4] = ld_cg_if(valid[s4], &ws.run[u[s4]]);
     }
+    bool ready[4];
 #pragma unroll
     for (int s4 = 0; s4 < 4; ++s4) {
-      const bool ready = valid[s4] && old4[s4] == 1u;
-      if (ready) {
+      ready[s4] = valid[s4] && old4[s4] == 1u;
+      if (ready[s4]) {
         ws.color[u[s4]] = next_color;
         ++coloured;
       }
-      push_ranges(ws, qs, hc_out, hcount_out, ready, wn[s4] > kHeavyDeg, u[s4], rb[s4], rb[s4] + wn[s4]);
     }
+    push_runs<4>(ws, q_out, hc_out, &ws.count[nxt], ready, run);
   };
   const uint32_t k = group_width(n, W.nwarps);
   WorkTaker lt((n + k - 1) / k, W.nwarps, ls, &ws.cursor[cur]);
@@ -688,13 +703,12 @@ __device__ __forceinline__ bool color_round(const GraphView& G, const Warps& W, 
     first = false;
     range_arcs4(rg.x, rg.y - rg.x, relax4);
   }
-  const uint32_t nch = (uint32_t)hp;
   WorkTaker ht(nch, W.nwarps, hs, &ws.hcursor[cur]);
   first = true;  // the first chunk taken is the warp's own, hs
   for (uint32_t c = ht.take(); c < nch; c = ht.take()) {
-    const uint4 ent = first ? hspec : ld_cg(&hc[c]);
+    const uint2 ent = first ? hspec : __ldcg(&hc[c]);
     first = false;
-    const uint32_t b = ent.y, en = ent.z;  // the entry's arc range
+    const uint32_t b = ent.x, en = ent.y;  // the entry's arc range
     // a chunk holds kChunk = 128 arcs: one four-step batch
     static_assert(kChunk == 4 * 32, "a colour chunk is one batch of four steps");
     bool valid[4];
@@ -706,7 +720,6 @@ __device__ __forceinline__ bool color_round(const GraphView& G, const Warps& W, 
     }
     relax4(valid, nullptr, arc);
   }
-  qs.flush();
   return true;
 }
 
@@ -715,19 +728,18 @@ __device__ __forceinline__ void color_body(Sync& s, const GraphView& G, const Co
   const Warps W = warps_of(s.id(), s.P());
   const bool leader = s.id() == 0 && threadIdx.x == 0;
   uint32_t* my = smem + (threadIdx.x & ~31u);  // smem: 2 x 512 words
-  __shared__ uint2 rstage[kMaxGraphWarps][64];  // per-warp queue staging
   unsigned long long arcs = 0, coloured = 0;
   color_init(G, W, ws);
   if (!s.sync()) return;
   color_count(G, ws, my, my + 512, arcs);
   if (!s.sync()) return;
-  color_first(G, W, ws, leader, rstage, coloured);
+  color_first(G, W, ws, leader, coloured);
   if (!s.sync()) return;
   // -- rounds: the vertices coloured in round r (queue slot r % 3) count
   // down the neighbours waiting for them
   uint32_t r = 1;
   for (;; ++r) {
-    if (!color_round(G, W, ws, r, leader, rstage, arcs, coloured)) break;
+    if (!color_round(G, W, ws, r, leader, arcs, coloured)) break;
     if (!s.sync()) return;
   }
 #pragma unroll
@@ -761,7 +773,6 @@ __global__ void k_color_rl_init(GraphView G, ColorWs ws) {
 __global__ void __launch_bounds__(512, 1) k_color_rl_step(GraphView G, ColorWs ws, StepCtl* ctl,
                                                          cudaGraphConditionalHandle cond) {
   __shared__ uint32_t smem[1024];
-  __shared__ uint2 rstage[kMaxGraphWarps][64];
   const StepCtl& st0 = step_state(ctl);
   const uint32_t kind = st0.s[0], r = st0.s[1];
   const Warps W = warps_of(blockIdx.x, gridDim.x);
@@ -770,9 +781,9 @@ __global__ void __launch_bounds__(512, 1) k_color_rl_step(GraphView G, ColorWs w
   if (kind == 0)
     color_count(G, ws, smem + (threadIdx.x & ~31u), smem + 512 + (threadIdx.x & ~31u), arcs);
   else if (kind == 1)
-    color_first(G, W, ws, leader, rstage, coloured);
+    color_first(G, W, ws, leader, coloured);
   else
-    color_round(G, W, ws, r, leader, rstage, arcs, coloured);
+    color_round(G, W, ws, r, leader, arcs, coloured);
   arcs = warp_add_u64(arcs);
   coloured = warp_add_u64(coloured);
   if (lane_id() == 0 && arcs) atomicAdd(&ws.stats[0], arcs);
@@ -785,7 +796,7 @@ __global__ void __launch_bounds__(512, 1) k_color_rl_step(GraphView G, ColorWs w
     // the next round's entries (slot r + 1), filled by this superstep
     const uint32_t nr = kind == 1 ? 1u : r + 1;
     const int nx = nr % 3;
-    const bool more = __ldcg(&ws.qcount[nx]) != 0 || __ldcg(&ws.hcount[nx]) != 0;
+    const bool more = __ldcg(&ws.count[nx]) != 0;
     st.s[0] = 2;
     st.s[1] = nr;
     if (!more) ws.stats[1] = nr - 1;
@@ -920,9 +931,9 @@ static int color_run(gdb_ctx* c, gdb_graph* g, const float* d_prio, int32_t* d_c
   Bump b;
   const size_t o_cnt_v = b.take((size_t)V * 4);
   const size_t o_q0 = b.take((size_t)V * 8), o_q1 = b.take((size_t)V * 8);
-  const size_t o_hc0 = b.take((size_t)hcap * 16), o_hc1 = b.take((size_t)hcap * 16);
+  const size_t o_hc0 = b.take((size_t)hcap * 8), o_hc1 = b.take((size_t)hcap * 8);
   const size_t o_wcol = b.take(std::max<uint64_t>(g->E, 1) * 4);
-  const size_t o_wcnt = b.take((size_t)V * 4);
+  const size_t o_run = b.take((size_t)V * 8);
   const size_t o_cnt = b.take(512);
   const size_t o_ctl = b.take(sizeof(StepCtl));
   char* base = (char*)workspace(c, b.off);
@@ -931,16 +942,15 @@ static int color_run(gdb_ctx* c, gdb_graph* g, const float* d_prio, int32_t* d_c
   ws.color = d_color;
   ws.cnt = (uint32_t*)(base + o_cnt_v);
   ws.wcol = (uint32_t*)(base + o_wcol);
-  ws.wcnt = (uint32_t*)(base + o_wcnt);
+  ws.run = (uint2*)(base + o_run);
   ws.prio = d_prio;
   ws.q[0] = (uint2*)(base + o_q0);
   ws.q[1] = (uint2*)(base + o_q1);
-  ws.hc[0] = (uint4*)(base + o_hc0);
-  ws.hc[1] = (uint4*)(base + o_hc1);
+  ws.hc[0] = (uint2*)(base + o_hc0);
+  ws.hc[1] = (uint2*)(base + o_hc1);
   char* cnt = base + o_cnt;
   ws.stats = (unsigned long long*)cnt;             // 4 x u64
-  ws.hcount = (unsigned long long*)(cnt + 64);     // 3 x u64
-  ws.qcount = (uint32_t*)(cnt + 96);
+  ws.count = (unsigned long long*)(cnt + 64);      // 3 x u64
   ws.cursor = (uint32_t*)(cnt + 112);
   ws.hcursor = (uint32_t*)(cnt + 128);
   ws.overflow = (int*)(cnt + 160);
@@ -950,7 +960,8 @@ static int color_run(gdb_ctx* c, gdb_graph* g, const float* d_prio, int32_t* d_c
   // after the count pass a round touches only the arcs of the vertices it
   // colours (thousands of small rounds on power-law graphs): latency-bound,
   // and faster on one CTA per SM (R-MAT-22: 42.8 ms against 47.4 ms on all
-  // 456 co-resident CTAs)
+  // 456 co-resident CTAs, measured before the batches took the registers that
+  // now leave room for one)
   // relaunched: the count pass, colour 1 and at most V rounds
   int rc = relaunch_kind(c) ? launch_steps(c, k_color_rl_init, k_color_rl_step, g->view(), ws, ws.stats,
                                            (StepCtl*)(base + o_ctl), StepCtl{}, (unsigned long long)V + 4,
