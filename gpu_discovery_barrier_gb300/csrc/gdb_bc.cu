@@ -952,17 +952,13 @@ static int bc_run(gdb_ctx* c, gdb_graph* g, const uint32_t* d_sources, uint32_t 
   k_bc_xf<<<s.grid, block, 0, c->stream>>>(a, g->view(), ws);
   GDB_CUDA(c, cudaGetLastError());
   GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  rc = finish_run(c);
+  int n = 0;
+  rc = finish_run(c, &n, cnt, 512);
   if (rc) return rc;
-  unsigned long long* hs = (unsigned long long*)pinned(c, 512);
-  if (!hs) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 512, cudaMemcpyDeviceToHost, c->stream));
-  GDB_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (*(int*)((char*)hs + 160)) return set_error(c, GDB_ERR_CAPACITY, "BC list overflow");
+  const unsigned long long* hs = (const unsigned long long*)pinned(c, 512);
+  if (*(const int*)((const char*)hs + 160)) return set_error(c, GDB_ERR_CAPACITY, "BC list overflow");
   float ms = 0;
   GDB_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-  int n = 0;
-  read_participating(c, &n);
   c->last.participating = n;
   c->last.launched = s.grid;
   c->last.launches = 1;

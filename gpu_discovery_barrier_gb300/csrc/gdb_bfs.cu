@@ -946,6 +946,7 @@ static int bfs_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_src
   const int kind = c->opt.barrier;
   c->last = gdb_run_stats{};
   int rc = GDB_OK;
+  bool counted = false;  // the counters came with the status
   if (kind == GDB_BARRIER_XF || kind == GDB_BARRIER_XF_FIXED) {
     Shape s;
     const void* kx = bfs_kernel(g, ws.adaptive, true, ws.queued != nullptr);
@@ -958,10 +959,10 @@ static int bfs_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_src
     ((BfsKernel)kx)<<<s.grid, block, smem, c->stream>>>(a, G, ws, src);
     GDB_CUDA(c, cudaGetLastError());
     GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-    rc = finish_run(c);
-    if (rc) return rc;
     int n = 0;
-    read_participating(c, &n);
+    rc = finish_run(c, &n, cnt, 512);
+    if (rc) return rc;
+    counted = true;
     c->last.participating = n;
     c->last.launched = s.grid;
     c->last.launches = 1;
@@ -1029,8 +1030,10 @@ static int bfs_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_src
   }
   unsigned long long* hs = (unsigned long long*)pinned(c, 512);
   if (!hs) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 512, cudaMemcpyDeviceToHost, c->stream));
-  GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (!counted) {
+    GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 512, cudaMemcpyDeviceToHost, c->stream));
+    GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  }
   if (*(int*)((char*)hs + 160)) return set_error(c, GDB_ERR_CAPACITY, "BFS queue overflow");
   float ms = 0;
   GDB_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));

@@ -827,16 +827,12 @@ static int launch_xf(gdb_ctx* c, K kernel, const GraphView& G, const Ws& ws, uns
   kernel<<<s.grid, block, 0, c->stream>>>(a, G, ws);
   GDB_CUDA(c, cudaGetLastError());
   GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  rc = finish_run(c);
+  int n = 0;
+  rc = finish_run(c, &n, d_stats, 16);
   if (rc) return rc;
-  unsigned long long* hs = (unsigned long long*)pinned(c, 64);
-  if (!hs) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hs, d_stats, 16, cudaMemcpyDeviceToHost, c->stream));
-  GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  const unsigned long long* hs = (const unsigned long long*)pinned(c, 64);
   float ms = 0;
   GDB_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-  int n = 0;
-  read_participating(c, &n);
   c->last.participating = n;
   c->last.launched = s.grid;
   c->last.launches = 1;

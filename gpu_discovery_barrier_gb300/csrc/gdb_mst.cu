@@ -433,12 +433,10 @@ static int mst_run(gdb_ctx* c, gdb_graph* g, gdb_mst_result* h_res, gdb_mst_resu
   k_mst_xf<<<s.grid, block, 0, c->stream>>>(a, g->view(), ws);
   GDB_CUDA(c, cudaGetLastError());
   GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-  rc = finish_run(c);
+  int n = 0;
+  rc = finish_run(c, &n, cnt, 128);
   if (rc) return rc;
-  unsigned long long* hs = (unsigned long long*)pinned(c, 256);
-  if (!hs) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 128, cudaMemcpyDeviceToHost, c->stream));
-  GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  const unsigned long long* hs = (const unsigned long long*)pinned(c, 256);
   if (*(const int*)((const char*)hs + 112))
     return set_error(c, GDB_ERR_INVALID, "MST: component pointers formed a cycle");
   gdb_mst_result r;
@@ -452,8 +450,6 @@ static int mst_run(gdb_ctx* c, gdb_graph* g, gdb_mst_result* h_res, gdb_mst_resu
   GDB_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0;
   GDB_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-  int n = 0;
-  read_participating(c, &n);
   c->last.participating = n;
   c->last.launched = s.grid;
   c->last.launches = 1;

@@ -1,5 +1,6 @@
 // libgdb host runtime: contexts, graphs, workspace, launch shapes, errors.
 #include <algorithm>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 
@@ -242,16 +243,25 @@ int run_on_lanes(gdb_ctx* c, uint32_t n, int lanes, bool fit_memory, size_t ws_b
 
 // Pinned staging layout: [0, 3072) run statistics of the callers,
 // [3072, 3584) participating count, [3584, 4096) device status.
-int finish_run(gdb_ctx* c) {
+int finish_run(gdb_ctx* c, int* participating, const void* d_words, size_t bytes) {
   char* base = (char*)pinned(c, 4096);
   if (!base) return set_error(c, GDB_ERR_OOM, "pinned staging");
-  int* h = (int*)(base + 3584);
-  // status, abort, err_where of the device context
-  GDB_CUDA(c, cudaMemcpyAsync(h, &c->dctx->status, 4 * sizeof(int), cudaMemcpyDeviceToHost,
-                              c->stream));
+  // num_participating to err_where of the device context: two lines
+  constexpr size_t kFrom = offsetof(gdb::DeviceCtx, num_participating);
+  constexpr size_t kTo = offsetof(gdb::DeviceCtx, err_where) + sizeof(int);
+  static_assert(kTo - kFrom <= 512, "the status words fit their place in the staging page");
+  char* h = base + 3584;
+  GDB_CUDA(c, cudaMemcpyAsync(h, (char*)c->dctx + kFrom, kTo - kFrom, cudaMemcpyDeviceToHost, c->stream));
+  if (bytes) GDB_CUDA(c, cudaMemcpyAsync(base, d_words, bytes, cudaMemcpyDeviceToHost, c->stream));
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return set_cuda_error(c, e, "kernel execution");
-  const int status = h[0], where = h[2];
+  auto word = [&](size_t at) {
+    int x;
+    std::memcpy(&x, h + at - kFrom, sizeof x);
+    return x;
+  };
+  const int status = word(offsetof(gdb::DeviceCtx, status)), where = word(offsetof(gdb::DeviceCtx, err_where));
+  if (participating) *participating = word(kFrom);
   if (status != 0) {
     int skip = 0;
     cudaMemcpy(&skip, &c->dctx->skip, sizeof(int), cudaMemcpyDeviceToHost);

@@ -1303,6 +1303,7 @@ static int sssp_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_sr
   GDB_CUDA(c, cudaMemsetAsync(cnt, 0, 512, c->stream));
   const int block = c->opt.block_size;
   c->last = gdb_run_stats{};
+  bool counted = false;  // the counters came with the status
   if (xf) {
     Shape s;
     auto kx = sssp_kernel(c, g, ws.delta, ws.light, ws.settle);
@@ -1313,10 +1314,10 @@ static int sssp_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_sr
     kx<<<s.grid, block, 0, c->stream>>>(a, GN, GH, GT, ws, src);
     GDB_CUDA(c, cudaGetLastError());
     GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-    rc = finish_run(c);
-    if (rc) return rc;
     int n = 0;
-    read_participating(c, &n);
+    rc = finish_run(c, &n, cnt, 512);
+    if (rc) return rc;
+    counted = true;
     c->last.participating = n;
     c->last.launched = s.grid;
   } else if (kind == GDB_BARRIER_GRID_SYNC) {
@@ -1381,8 +1382,10 @@ static int sssp_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_sr
     c->last.launches = 1;
   unsigned long long* hs = (unsigned long long*)pinned(c, 512);
   if (!hs) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 512, cudaMemcpyDeviceToHost, c->stream));
-  GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (!counted) {
+    GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 512, cudaMemcpyDeviceToHost, c->stream));
+    GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  }
   if (*(int*)((char*)hs + 160)) return set_error(c, GDB_ERR_CAPACITY, "SSSP queue overflow");
   float ms = 0;
   GDB_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
@@ -1425,7 +1428,7 @@ static int jacobi_run(gdb_ctx* c, gdb_graph* g, uint32_t src, int32_t* d_cost) {
   const int block = c->opt.block_size;
   c->last = gdb_run_stats{};
   Shape s;
-  int rc = GDB_OK;
+  int rc = GDB_OK, n = 0;
   if (relaunch) {
     int grid = 0;
     if ((rc = step_grid(c, (const void*)k_jacobi_rl_step, block, &grid))) return rc;
@@ -1443,14 +1446,17 @@ static int jacobi_run(gdb_ctx* c, gdb_graph* g, uint32_t src, int32_t* d_cost) {
     k_jacobi_xf<<<s.grid, block, 0, c->stream>>>(a, G, ws, src);
     GDB_CUDA(c, cudaGetLastError());
     GDB_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-    rc = finish_run(c);
+    rc = finish_run(c, &n, cnt, 64);
     if (rc) return rc;
   }
   const uint32_t launches = relaunch ? c->last.launches : 1;
   unsigned long long* hs = (unsigned long long*)pinned(c, 256);
   if (!hs) return GDB_ERR_OOM;
-  GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 64, cudaMemcpyDeviceToHost, c->stream));
-  GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (relaunch) {
+    n = s.grid;
+    GDB_CUDA(c, cudaMemcpyAsync(hs, cnt, 64, cudaMemcpyDeviceToHost, c->stream));
+    GDB_CUDA(c, cudaStreamSynchronize(c->stream));
+  }
   const uint32_t k = (uint32_t)hs[1];
   if (k >= 1 && ((k - 1) & 1)) {
     GDB_CUDA(c, cudaMemcpyAsync(d_cost, ws.x[1], (size_t)g->V * 4, cudaMemcpyDeviceToDevice, c->stream));
@@ -1459,8 +1465,6 @@ static int jacobi_run(gdb_ctx* c, gdb_graph* g, uint32_t src, int32_t* d_cost) {
   GDB_CUDA(c, cudaStreamSynchronize(c->stream));
   float ms = 0;
   GDB_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-  int n = s.grid;
-  if (!relaunch) read_participating(c, &n);
   c->last.participating = n;
   c->last.launched = s.grid;
   c->last.launches = launches;
