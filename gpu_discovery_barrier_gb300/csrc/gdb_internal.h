@@ -120,6 +120,15 @@ struct Shape {
 
 int persistent_shape(gdb_ctx* c, const void* kernel, int block, size_t smem, Shape* s,
                      bool allow_oversubscribe = true);
+// One CTA per SM for a traversal of a small graph, alone on the GPU and with
+// the shape left open: discovery and every barrier wait for fewer CTAs, and
+// its supersteps do not fill the warps of one per SM.  All co-resident CTAs
+// against one per SM, whole calls in us: R-MAT 1,000 vertices (16 k arcs)
+// BFS 83 / 80, SSSP 107 / 98.5; 20,000 (300 k) 117 / 108, 202 / 191; grid of
+// 150,000 (600 k) 739 / 738, 1104 / 1096; the line is eight arcs per thread
+// (622 k), since the grid of 400,000 (1.6 M) loses: SSSP 1873 / 2079, its
+// hops spread over fewer CTAs.
+void small_shape(gdb_ctx* c, const gdb_graph* g, Shape* s);
 gdb::DiscoveryArgs discovery_args(gdb_ctx* c, const Shape& s);
 
 // After a persistent run: wait for it and read the device status, and with

@@ -73,6 +73,11 @@ int persistent_shape(gdb_ctx* c, const void* kernel, int block, size_t smem, Sha
   return GDB_OK;
 }
 
+void small_shape(gdb_ctx* c, const gdb_graph* g, Shape* s) {
+  if (c->opt.max_ctas > 0 || c->opt.oversubscribe > 0 || c->cap_override > 0) return;
+  if (g->E <= (uint64_t)c->sm_count * s->block * 8) s->grid = std::min(s->grid, c->sm_count);
+}
+
 gdb::DiscoveryArgs discovery_args(gdb_ctx* c, const Shape& s) {
   gdb::DiscoveryArgs a;
   a.ctx = c->dctx;
