@@ -412,32 +412,6 @@ struct ColorWs {
 // then has two entries in turn), starting on the entries before the counts are
 // known (14.5), writing the colours one batch later (14.1).
 
-// Loads and count-downs under a predicate, as single instructions.  Written
-// as conditional expressions they became branches, and lanes that had parted
-// there went through the batch one group after the other, each with its own
-// round trips.
-__device__ __forceinline__ uint32_t ld_cg_if(bool p, const uint32_t* a) {
-  uint32_t x;
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; mov.u32 %0, 0; @p ld.global.cg.u32 %0, [%1]; }"
-               : "=r"(x) : "l"(a), "r"((uint32_t)p) : "memory");
-  return x;
-}
-__device__ __forceinline__ uint2 ld_cg_if(bool p, const uint2* a) {
-  uint2 x;
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %3, 0; mov.u32 %0, 0; mov.u32 %1, 0;\n"
-               " @p ld.global.cg.v2.u32 {%0, %1}, [%2]; }"
-               : "=r"(x.x), "=r"(x.y) : "l"(a), "r"((uint32_t)p) : "memory");
-  return x;
-}
-// *a - 1 under p, returning what it was (0 without p)
-__device__ __forceinline__ uint32_t count_down_if(bool p, uint32_t* a) {
-  uint32_t x;
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; mov.u32 %0, 0;\n"
-               " @p atom.global.add.u32 %0, [%1], -1; }"
-               : "=r"(x) : "l"(a), "r"((uint32_t)p) : "memory");
-  return x;
-}
-
 // Push the lanes' ready vertices of N steps, with their runs: a light one
 // (at most kHeavyDeg wait for it) as one entry, a heavy one as chunks.  One
 // reservation for both lists and all steps.

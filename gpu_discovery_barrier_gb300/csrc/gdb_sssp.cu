@@ -832,13 +832,21 @@ __device__ __forceinline__ bool jacobi_iter(const GraphView& G, const JacobiWs& 
     bool hit[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      u[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
+      u[j] = ldg_if(valid[j], &G.col[arc[j]]);
       arcs += valid[j];
     }
+    uint32_t word[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) hit[j] = valid[j] && (k == 0 || ((in[u[j] >> 5] >> (u[j] & 31)) & 1u));
+    for (int j = 0; j < 4; ++j) word[j] = ld_if(valid[j] && k != 0, &in[u[j] >> 5]);
+    uint32_t w[4], x[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) c[j] = hit[j] ? (int32_t)(__ldg(&G.w[arc[j]]) + (uint32_t)xo[u[j]]) : INT32_MAX;
+    for (int j = 0; j < 4; ++j) {
+      hit[j] = valid[j] && (k == 0 || ((word[j] >> (u[j] & 31)) & 1u));
+      w[j] = ldg_if(hit[j], &G.w[arc[j]]);
+      x[j] = ld_if(hit[j], &xo[u[j]]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[j] = hit[j] ? (int32_t)(w[j] + x[j]) : INT32_MAX;
   };
   sweep_light4(
       G, &ws.cursor[cur],
