@@ -1237,9 +1237,14 @@ static int settle_of(const gdb_ctx* c, uint32_t light, int force) {
 // arcs per vertex on average, and graphs whose every frontier is small.
 // What is left to k_sssp_xf besides the split is the plain worklist on
 // R-MAT-like graphs, a dozen wide supersteps that the narrow kernel's shared
-// memory slows (R-MAT-22 3.93 -> 4.0 to 4.1 ms per source).
+// memory slows (R-MAT-22 3.93 -> 4.0 to 4.1 ms per source), and the plain
+// worklist on the largest thin graphs, whose frontiers are wide for most of
+// the run and which a CTA's own order makes relax a tenth more arcs: grids
+// of 16.8 M vertices 480 -> 503 ms, 12.3 M 306 -> 300, 12.0 M (12,000 rows)
+// 1488 -> 1458, 8.4 M 194 -> 169, 1 M 29 -> 5.
+constexpr uint32_t kNarrowPlainV = 12u << 20;
 static auto sssp_kernel(const gdb_ctx* c, const gdb_graph* g, uint32_t delta, uint32_t light, int settle) {
-  const bool narrow = light >= kInf && (delta > 0 || g->E <= 8ull * g->V ||
+  const bool narrow = light >= kInf && (delta > 0 || (g->E <= 8ull * g->V && g->V <= kNarrowPlainV) ||
                                         g->V <= (uint64_t)c->sm_count * drain_share(g->E, g->V, SsspDrain::kCap));
   return settle != kSettleRule ? k_sssp_xf_sel : narrow ? k_sssp_xf_narrow : k_sssp_xf;
 }
