@@ -132,8 +132,9 @@ def alg_bytes(app: str, g, reached, rounds: int) -> float:
     """Algorithmic bytes of one launch (uint32 = 4 B), schedule-independent:
     BFS 8E_r + 12V_r + 4V; SSSP 12E_r + 12V_r + 4V; BC 20E_r + 24V_r + 12V
     per source; MST (12E + 16V) per round; colouring 24E + 16V (one count
-    pass and one countdown pass over the arcs); MIS (12E + 8V) per round,
-    bounded from above by the full graph."""
+    pass and one countdown pass over the arcs); MIS 4E once, bounded from
+    above by the full graph (a vertex stops at the first neighbour that beats
+    it), and 8V per round."""
     V, E = g.V, g.E
     if app == "bfs":
         return sum(8 * er + 12 * vr + 4 * V for vr, er in reached)
@@ -147,7 +148,7 @@ def alg_bytes(app: str, g, reached, rounds: int) -> float:
         # count pass (col + neighbour priority per arc) and one countdown
         # pass (col, neighbour degree and priority, counter) per arc
         return 8 * E + 8 * V + 16 * E + 8 * V
-    return rounds * (12 * E + 8 * V)
+    return 4 * E + rounds * 8 * V
 
 
 def peaks():
