@@ -954,7 +954,7 @@ static int bfs_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_src
     bfs_bitmap(c, g, &ws, true, &smem);
     rc = persistent_shape(c, kx, block, smem, &s, kind == GDB_BARRIER_XF);
     if (rc) return rc;
-    small_shape(c, g, &s);
+    if (force < 0) small_shape(c, g, &s);  // traces time the shape they ask for
     DiscoveryArgs a = discovery_args(c, s);
     GDB_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     ((BfsKernel)kx)<<<s.grid, block, smem, c->stream>>>(a, G, ws, src);

@@ -1322,7 +1322,7 @@ static int sssp_run(gdb_ctx* c, gdb_graph* g, uint32_t src, const uint32_t* d_sr
     auto kx = sssp_kernel(c, g, ws.delta, ws.light, ws.settle);
     rc = persistent_shape(c, (const void*)kx, block, 0, &s, kind == GDB_BARRIER_XF);
     if (rc) return rc;
-    small_shape(c, g, &s);
+    if (force_settle < 0) small_shape(c, g, &s);
     DiscoveryArgs a = discovery_args(c, s);
     GDB_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     kx<<<s.grid, block, 0, c->stream>>>(a, GN, GH, GT, ws, src);
