@@ -606,9 +606,9 @@ __device__ __forceinline__ void sssp_body(Sync& s, const GraphView& G, const Gra
     const bool dry = sc[0] == 0 && sc[1] == 0;
     const uint32_t sn = (uint32_t)sc[4], hn = (uint32_t)sc[5];
     const bool unsettled = !Narrow && (sn > sdone || hn > hdone);
+    if (leader && narrow) inner += max(ld_cg(&ws.cursor[old]), 1u) - 1u;  // the last superstep's too
     if (dry && !unsettled && (!ws.delta || sc[2] == 0)) break;
     if (leader) {
-      if (narrow) inner += max(ld_cg(&ws.cursor[old]), 1u) - 1u;
       ws.qcount[old] = 0;
       ws.hcount[old] = 0;
       ws.cursor[old] = 0;
