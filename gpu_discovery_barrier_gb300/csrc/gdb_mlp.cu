@@ -5,7 +5,7 @@
 //   k_mlp_grad  a CTA takes tiles of 128 samples: forward and backward pass
 //               into shared memory, then the tile's share of every gradient
 //               entry from there (register tiles of 4 x 4 entries), kept in
-//               registers from tile to tile as a pair of floats;
+//               FP64 registers from tile to tile;
 //   k_mlp_step  one warp per gradient entry: the CTAs' sums in a fixed order
 //               in FP64, then the Adam update of that parameter.
 // Tiles, lanes and sums have a fixed order, so gradients are bit-identical
@@ -84,13 +84,6 @@ constexpr int kMlpThreads = 256;
 constexpr int kMlpSmem = (kRows * kPitch + ((kRows + 3) & ~3) + ((kParams + 3) & ~3)) * 4;
 static_assert(kPW1 % 4 == 0 && kPW2 % 4 == 0, "weight rows are read as float4");
 
-// Exact-to-2^-48 accumulation of one more term into the pair (hi, lo).
-__device__ __forceinline__ void pair_add(float& hi, float& lo, float x) {
-  const float t = __fadd_rn(hi, x), z = __fsub_rn(t, hi);
-  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(x, z)));
-  hi = t;
-}
-
 // Forward pass, errors and gradient sums of the CTA's tiles.  The gradient
 // is the contraction of activation rows with error rows over the samples.
 // It was one warp per entry with an FP64 FMA per (entry, sample) and both
@@ -150,9 +143,11 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
   auto drow = [&](int j) { return j < 3 ? j * ds : d3; };
   const int colr0 = tid - 208, colr1 = colr0 + 48;  // column sums: rows of dh1, dh2, dy, loss from kRDh1
   constexpr int kCols = kRows - kRDh1;
-  float rhi[16], rlo[16];
+  // sums over the CTA's tiles, in FP64: partial sums beyond the floats' range
+  // stay finite, and infinite terms stay infinite
+  double sum[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) rhi[i] = rlo[i] = 0.f;
+  for (int i = 0; i < 16; ++i) sum[i] = 0.0;
 
   for (uint32_t tile = blockIdx.x; (size_t)tile * kTile < n; tile += gridDim.x) {
     const size_t base = (size_t)tile * kTile;
@@ -331,20 +326,18 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int e = 4 * i + j;
-            pair_add(rhi[e], rlo[e], __fsub_rn(acc[e], grid_of(i, j)));
-            pair_add(rhi[e], rlo[e], lo[e]);
+            sum[e] += (double)__fsub_rn(acc[e], grid_of(i, j)) + (double)lo[e];
           }
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            double sum = 0.0;
+            const float *x = A + i * as * kPitch, *y = D + drow(j) * kPitch;
+            double t = 0.0;
 #pragma unroll 1
-            for (int s = 0; s < 64; ++s) sum += (double)A[i * as * kPitch + s] * (double)D[drow(j) * kPitch + s];
-            const float f = (float)sum;
-            pair_add(rhi[4 * i + j], rlo[4 * i + j], f);
-            pair_add(rhi[4 * i + j], rlo[4 * i + j], (float)(sum - (double)f));
+            for (int s = 0; s < 64 && 64 * half + s < (int)have; ++s) t += (double)x[s] * (double)y[s];
+            sum[4 * i + j] += t;
           }
       }
     } else {
@@ -352,8 +345,8 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
       const float* c1 = act + (kRDh1 + (colr1 < kCols ? colr1 : colr0)) * kPitch;
 #pragma unroll 4
       for (int s = 0; s < kTile; ++s) {
-        pair_add(rhi[0], rlo[0], c0[s]);
-        pair_add(rhi[1], rlo[1], c1[s]);
+        sum[0] += (double)c0[s];
+        sum[1] += (double)c1[s];
       }
     }
   }
@@ -365,8 +358,7 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (j < nd)
-          part[(size_t)(out0 - kPW1 + i * outw + j * ocol) * slots + 2 * blockIdx.x + half] =
-              (double)rhi[4 * i + j] + (double)rlo[4 * i + j];
+          part[(size_t)(out0 - kPW1 + i * outw + j * ocol) * slots + 2 * blockIdx.x + half] = sum[4 * i + j];
   } else {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -376,7 +368,7 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
       const int e = c < kH1 ? kPB1 + c : c < kH1 + kH2 ? kPB2 + c - kH1
                   : c < kH1 + kH2 + kOut ? kPB3 + c - kH1 - kH2 : kParams;
       double* o = part + (size_t)(e - kPW1) * slots + 2 * blockIdx.x;
-      o[0] = (double)rhi[k] + (double)rlo[k];
+      o[0] = sum[k];
       o[1] = 0.0;
     }
   }
