@@ -84,6 +84,19 @@ constexpr int kMlpThreads = 256;
 constexpr int kMlpSmem = (kRows * kPitch + ((kRows + 3) & ~3) + ((kParams + 3) & ~3)) * 4;
 static_assert(kPW1 % 4 == 0 && kPW2 % 4 == 0, "weight rows are read as float4");
 
+// a + b; err: what rounding took from it, exactly.
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float t = __fadd_rn(a, b), z = __fsub_rn(t, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
+  return t;
+}
+
+// Largest magnitude of a product or column value that a run of floats takes
+// (2^32 values on 304 CTAs stay below 1e36), and the tiles of
+// a run of products.
+constexpr float kRunMax = 1e28f;
+constexpr uint32_t kRunTiles = 8;
+
 // Forward pass, errors and gradient sums of the CTA's tiles.  The gradient
 // is the contraction of activation rows with error rows over the samples.
 // It was one warp per entry with an FP64 FMA per (entry, sample) and both
@@ -92,16 +105,19 @@ static_assert(kPW1 % 4 == 0 && kPW2 % 4 == 0, "weight rows are read as float4");
 //  * the rows stay in shared memory: a thread holds 4 x 4 entries and reads
 //    eight 16-byte row pieces per four samples; tiles' rows interleave (t,
 //    t + 8, ...), so a warp's eight distinct rows fall on distinct banks;
-//  * FP64's place is taken by error-free extraction against a fixed grid
-//    (Rump, Ogita, Oishi, "Accurate floating-point summation", SIAM J. Sci.
-//    Comput. 31(1), 2008): with C = 1.5 x 2^k above the sum of the tile's
-//    |products| (from the rows' largest magnitudes), acc = fma(a, b, acc)
-//    rounds a product onto C's grid, acc' - acc is that part exactly, and
-//    fma(a, b, -part) the rest, which goes to a second float.  Four FP32
-//    operations per product, an error near 2^-35 of the largest product
-//    (below the 2^-24 of the float gradient).  Where the grid would
-//    overflow, the thread sums its tile in FP64 instead.
-// 135,000 samples: 1.9 -> 0.11 ms a step, k_mlp_step included.
+//  * FP64's place is taken by pairs of floats (Ogita, Rump, Oishi, "Accurate
+//    sum and dot product", SIAM J. Sci. Comput. 26(6), 2005): p = a b and its
+//    error fma(a, b, -p), hi + p and its error, both errors into lo.  Ten
+//    FP32 operations per product, each exact but the adds into lo: measured
+//    against 64 bits, a run of 64 products is within 2^-43 of the sum of
+//    their magnitudes and one of 1,024 within 2^-39, whatever the rows' other
+//    values are, and rounded to a float both are what FP64 sums give
+//    (products below 2^-102 lose up to 2^-150 each).  Runs of kRunTiles tiles
+//    go to FP64 sums in global memory.  The column sums (biases, loss) are
+//    triples, beyond FP64's 53 bits.
+//    Where a product or a value could bring a run near the floats' range, or
+//    is not finite, the thread takes its tile in FP64 instead.
+// 135,000 samples: 1.9 -> 0.17 ms a step, k_mlp_step included.
 __global__ void __launch_bounds__(kMlpThreads, 2)
     k_mlp_grad(const float* __restrict__ p, const float* __restrict__ X, const float* __restrict__ T,
                const float* __restrict__ M, uint32_t n, const float* __restrict__ inv_mask,
@@ -143,11 +159,38 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
   auto drow = [&](int j) { return j < 3 ? j * ds : d3; };
   const int colr0 = tid - 208, colr1 = colr0 + 48;  // column sums: rows of dh1, dh2, dy, loss from kRDh1
   constexpr int kCols = kRows - kRDh1;
-  // sums over the CTA's tiles, in FP64: partial sums beyond the floats' range
-  // stay finite, and infinite terms stay infinite
-  double sum[16];
+  // products: the run's pair of entry 4 i + j; columns: hi[k], lo[k], hi[2 + k]
+  // are column k's triple
+  float hi[16], lo[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) sum[i] = 0.0;
+  for (int i = 0; i < 16; ++i) hi[i] = lo[i] = 0.f;
+  // part[entry][slot]: two slots per CTA, one per half of the samples.  put
+  // adds a sum to this thread's slot of an entry; `begun`: slots hold one
+  const size_t slots = 2 * (size_t)gridDim.x;
+  double* mine = part + 2 * blockIdx.x + (tiled ? half : 0);
+  bool begun = false;
+  auto put = [&](int entry, double x) {
+    double* o = mine + (size_t)entry * slots;
+    *o = begun ? *o + x : x;
+  };
+  auto entry = [&](int i, int j) { return out0 - kPW1 + i * outw + j * ocol; };
+  // column c's entry: dh1, dh2 and dy are the biases; the loss is the last one
+  auto column = [&](int c) {
+    return (c < kH1 ? kPB1 + c : c < kH1 + kH2 ? kPB2 + c - kH1 : c < kH1 + kH2 + kOut ? kPB3 + c - kH1 - kH2 : kParams) -
+           kPW1;
+  };
+  auto end_run = [&] {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int e = 4 * i + j;
+        if (j < nd) put(entry(i, j), (double)hi[e] + (double)lo[e]);
+        hi[e] = lo[e] = 0.f;
+      }
+    begun = true;
+  };
+  uint32_t run = 0;
 
   for (uint32_t tile = blockIdx.x; (size_t)tile * kTile < n; tile += gridDim.x) {
     const size_t base = (size_t)tile * kTile;
@@ -279,22 +322,11 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
     }
     __syncthreads();
     if (tiled) {
-      // C = 1.5 x 2^k with 2^k above twice the largest possible |sum| of
-      // the 64 products, so acc keeps C's exponent throughout
-      auto grid_of = [&](int i, int j) {
-        const float b = top[a0 + i * as] * top[d0 + drow(j)] * 160.f;
-        return 1.5f * __uint_as_float((__float_as_uint(b) & 0x7f800000u) + 0x00800000u);
-      };
       bool fits = true;
-      float acc[16], lo[16];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          fits = fits && top[a0 + i * as] * top[d0 + drow(j)] < 1e34f;
-          acc[4 * i + j] = grid_of(i, j);
-          lo[4 * i + j] = 0.f;
-        }
+        for (int j = 0; j < 4; ++j) fits = fits && top[a0 + i * as] * top[d0 + drow(j)] < kRunMax;
       const float* A = act + a0 * kPitch + 64 * half;
       const float* D = act + d0 * kPitch + 64 * half;
       if (fits) {
@@ -315,19 +347,16 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const int e = 4 * i + j;
-                const float t = __fmaf_rn(av[i][q], dv[j][q], acc[e]);
-                const float on = __fsub_rn(t, acc[e]);
-                lo[e] = __fadd_rn(lo[e], __fmaf_rn(av[i][q], dv[j][q], -on));
-                acc[e] = t;
+                const float t = __fmul_rn(av[i][q], dv[j][q]);
+                float err;
+                hi[e] = two_sum(hi[e], t, err);
+                lo[e] = __fadd_rn(lo[e], __fadd_rn(err, __fmaf_rn(av[i][q], dv[j][q], -t)));
               }
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int e = 4 * i + j;
-            sum[e] += (double)__fsub_rn(acc[e], grid_of(i, j)) + (double)lo[e];
-          }
+        if (++run == kRunTiles) {
+          end_run();
+          run = 0;
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -337,39 +366,44 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
             double t = 0.0;
 #pragma unroll 1
             for (int s = 0; s < 64 && 64 * half + s < (int)have; ++s) t += (double)x[s] * (double)y[s];
-            sum[4 * i + j] += t;
+            if (j < nd) put(entry(i, j), t);
           }
+        begun = true;
       }
-    } else {
+    } else if (top[kRDh1 + colr0] < kRunMax && !(colr1 < kCols && !(top[kRDh1 + colr1] < kRunMax))) {
       const float* c0 = act + (kRDh1 + colr0) * kPitch;
       const float* c1 = act + (kRDh1 + (colr1 < kCols ? colr1 : colr0)) * kPitch;
 #pragma unroll 4
-      for (int s = 0; s < kTile; ++s) {
-        sum[0] += (double)c0[s];
-        sum[1] += (double)c1[s];
+      for (int s = 0; s < kTile; ++s)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          float e0, e1;
+          hi[k] = two_sum(hi[k], k ? c1[s] : c0[s], e0);
+          lo[k] = two_sum(lo[k], e0, e1);
+          hi[2 + k] = __fadd_rn(hi[2 + k], e1);
+        }
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) {
+        const int c = k ? colr1 : colr0;
+        if (c >= kCols) break;
+        const float* x = act + (kRDh1 + c) * kPitch;
+        double t = 0.0;
+        for (uint32_t s = 0; s < have; ++s) t += (double)x[s];
+        put(column(c), t);
       }
+      begun = true;
     }
   }
-  // part[entry][slot]: two slots per CTA, one per half of the samples
-  const size_t slots = 2 * (size_t)gridDim.x;
   if (tiled) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < nd)
-          part[(size_t)(out0 - kPW1 + i * outw + j * ocol) * slots + 2 * blockIdx.x + half] = sum[4 * i + j];
+    end_run();
   } else {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int c = k ? colr1 : colr0;
       if (c >= kCols) break;
-      // dh1, dh2 and dy columns are the biases; the loss is the last entry
-      const int e = c < kH1 ? kPB1 + c : c < kH1 + kH2 ? kPB2 + c - kH1
-                  : c < kH1 + kH2 + kOut ? kPB3 + c - kH1 - kH2 : kParams;
-      double* o = part + (size_t)(e - kPW1) * slots + 2 * blockIdx.x;
-      o[0] = sum[k];
-      o[1] = 0.0;
+      put(column(c), (double)hi[k] + ((double)lo[k] + (double)hi[2 + k]));
+      mine[(size_t)column(c) * slots + 1] = 0.0;
     }
   }
 }
