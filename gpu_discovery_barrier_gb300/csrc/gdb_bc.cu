@@ -54,7 +54,8 @@ using namespace gdb;
 // sectors, and pulls are bound by those).  Coefficients of levels above the
 // peak are pushed, never read, and not stored, so a count stays readable for
 // every chunk of a heavy vertex there.  sacc: FP64 accumulator of the
-// backward sum of pushed levels.
+// backward sum of pushed levels, and before that of a heavy vertex's pulled
+// path count; -0.0 when it holds neither.
 // The pulls' and the backward pushes' loads of st are ordinary ones, through
 // L1: what they look for was final at the last barrier, whose acquire drops
 // older lines, and a stale level of a vertex being claimed is not the one
@@ -67,6 +68,7 @@ struct BcWs {
   uint4* hc;                     // heavy chunk entries, level segments
   double* hacc;                  // FP64 partial sums per heavy vertex slot
   uint32_t* hleft;               // chunks still to finish per heavy vertex slot
+  uint32_t* hpull;               // chunks summed in a forward pull, per heavy index; 0 between levels
   uint32_t hc_cap;               // chunk entries available
   uint32_t* lev_l;               // light segment start per level
   uint32_t* lev_h;               // heavy chunk-entry start per level
@@ -155,6 +157,25 @@ __device__ __forceinline__ void chunk_steps(uint32_t b, uint32_t e, bool* valid,
   }
 }
 
+// Sums over the warp of four values per lane: lane l returns that of
+// x[l / 8], six shuffles for the four.
+__device__ __forceinline__ float four_sums(const float* x) {
+  const bool b16 = lane_id() & 16, b8 = lane_id() & 8;
+  const float y0 = (b16 ? x[2] : x[0]) + __shfl_xor_sync(kFull, b16 ? x[0] : x[2], 16);
+  const float y1 = (b16 ? x[3] : x[1]) + __shfl_xor_sync(kFull, b16 ? x[1] : x[3], 16);
+  float z = (b8 ? y1 : y0) + __shfl_xor_sync(kFull, b8 ? y0 : y1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(kFull, z, o);
+  return z;
+}
+
+// a + b; err: what rounding took from it, exactly (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float t = __fadd_rn(a, b), z = __fsub_rn(t, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
+  return t;
+}
+
 __device__ __forceinline__ int32_t level_of(const BcWs& ws, uint32_t v) {
   return (int32_t)__ldcg(reinterpret_cast<const uint32_t*>(&ws.st[v]));
 }
@@ -224,6 +245,7 @@ __device__ __forceinline__ void bc_init(const GraphView& G, const Warps& W, cons
     ws.sacc[v] = -0.0;
     ws.bc[v] = 0.f;
   }
+  for (uint32_t h = W.gthread; h < G.nheavy; h += W.nthreads) ws.hpull[h] = 0;
   if (leader) {
     for (int i = 0; i < 3; ++i) {
       ws.lcnt[i] = 0;
@@ -404,45 +426,70 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
       frontier_push_staged(G, out, qs, claimed, u);
     });
     // the unvisited heavy vertices chunk by chunk (a hub left to one warp
-    // held the level up for hundreds of microseconds): the first chunk with
-    // a parent claims the vertex, each adds its FP32 sum as a push would
+    // held the level up for hundreds of microseconds).  Accumulated as a
+    // light vertex's count is: FP32 over a 32-arc step, then beyond floats --
+    // a pair per step of the warp's successive chunks of one vertex, FP64
+    // over the warps in sacc, which the forward pass leaves idle -- and
+    // rounded once, by the warp that brings the vertex's last chunk, which
+    // also claims it.  (FP32 atomics of the chunks' sums lost what stays
+    // under half a unit of a hub's count, and depended on their order.)
     while (nhvbase < G.nheavy) {  // some left
       const uint32_t base = warp_grab(&ws.hcursor[cur]) * 32;
       if (base >= G.nheavy_chunks) break;
       const uint4 ent = base + lane < G.nheavy_chunks ? __ldg(&G.heavy_chunk[base + lane]) : make_uint4(0, 0, 0, 0);
-      // L + 1: claimed by another chunk in this superstep
-      const int32_t lu = ent.w ? level_of(ws, ent.x) : -2;
-      const bool open = lu == -1 || lu == Li + 1;
+      const bool open = ent.w && level_of(ws, ent.x) == -1;  // until its last chunk is in
       uint32_t rb = 0, re = 0;
       if (open) {
         rb = __ldg(&G.row[ent.x]) + ent.y * kChunk;
         re = min(__ldg(&G.row[ent.x + 1]), rb + kChunk);
       }
+      float hi = 0.f, lo = 0.f;  // of step lane / 8
+      uint32_t run = 0;          // chunks summed
       for (unsigned todo = __ballot_sync(kFull, open); todo; todo &= todo - 1) {
         const int o = __ffs(todo) - 1;
         const uint32_t u = __shfl_sync(kFull, ent.x, o);
         bool valid[4];
         uint32_t arc[4], w[4];
         uint2 sw[4];
+        float x[4];
         chunk_steps(__shfl_sync(kFull, rb, o), __shfl_sync(kFull, re, o), valid, arc);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           w[j] = valid[j] ? __ldg(&G.col[arc[j]]) : 0u;
           arcs += valid[j];
         }
-        float part = 0.f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) sw[j] = valid[j] ? ws.st[w[j]] : kUnreached;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) part += (int32_t)sw[j].x == Li ? __uint_as_float(sw[j].y) : 0.f;
-        part = warp_sum_f32(part);
+        for (int j = 0; j < 4; ++j) x[j] = (int32_t)sw[j].x == Li ? __uint_as_float(sw[j].y) : 0.f;
+        float err;
+        hi = two_sum(hi, four_sums(x), err);
+        lo += err;
+        ++run;
+        const unsigned rest = todo & (todo - 1);
+        if (rest && __shfl_sync(kFull, ent.x, __ffs(rest) - 1) == u) continue;
+        double part = isinf(hi) ? (double)hi : (double)hi + (double)lo;
+        part += __shfl_xor_sync(kFull, part, 8);
+        part += __shfl_xor_sync(kFull, part, 16);
+        const uint32_t h = __shfl_sync(kFull, ent.z, o), nchunks = __shfl_sync(kFull, ent.w, o);
         bool claimed = false;
-        if (lane == 0 && part > 0.f) {
-          claimed = atomicCAS(reinterpret_cast<int*>(&ws.st[u].x), -1, Li + 1) == -1;
-          atomicAdd(reinterpret_cast<float*>(&ws.st[u].y), part);
-          if (claimed) next_arcs += degree(u);
+        if (lane == 0) {
+          if (part > 0.0) atomicAdd(&ws.sacc[u], part);
+          // as in heavy_done: the last one reads every warp's add
+          if (add_acq_rel(&ws.hpull[h], run) + run == nchunks) {
+            const double sum = __ldcg(&ws.sacc[u]);
+            ws.hpull[h] = 0;
+            claimed = sum > 0.0;
+            if (claimed) {
+              ws.sacc[u] = -0.0;
+              ws.st[u] = make_uint2((uint32_t)(Li + 1), __float_as_uint((float)sum));
+              next_arcs += degree(u);
+            }
+          }
         }
         if (__any_sync(kFull, claimed)) frontier_push_staged(G, out, qs, claimed, u);
+        hi = lo = 0.f;
+        run = 0;
       }
     }
     if (leader) reached_arcs += mf;
@@ -802,7 +849,7 @@ static size_t bc_layout(const gdb_graph* g, char* base, float* d_bc, const uint3
   const size_t o_st = b.take((size_t)V * 8), o_sacc = b.take((size_t)V * 8);
   const size_t o_ord = b.take((size_t)V * 4);
   const size_t o_hc = b.take((size_t)ccap * 16), o_hacc = b.take((size_t)hcap * 8),
-               o_hleft = b.take((size_t)hcap * 4);
+               o_hleft = b.take((size_t)hcap * 4), o_hpull = b.take((size_t)hcap * 4);
   const size_t o_ll = b.take((size_t)maxlev * 4), o_lh = b.take((size_t)maxlev * 4),
                o_lhc = b.take((size_t)maxlev * 4), o_lhv = b.take((size_t)maxlev * 4);
   const size_t o_la = b.take((size_t)(maxlev + 2) * 8);
@@ -816,6 +863,7 @@ static size_t bc_layout(const gdb_graph* g, char* base, float* d_bc, const uint3
   ws->hc_cap = ccap;
   ws->hacc = (double*)(base + o_hacc);
   ws->hleft = (uint32_t*)(base + o_hleft);
+  ws->hpull = (uint32_t*)(base + o_hpull);
   ws->lev_l = (uint32_t*)(base + o_ll);
   ws->lev_h = (uint32_t*)(base + o_lh);
   ws->lev_hc = (uint32_t*)(base + o_lhc);

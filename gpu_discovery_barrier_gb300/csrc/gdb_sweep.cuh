@@ -691,14 +691,15 @@ __device__ __forceinline__ const unsigned long long* cta_words(Load&& load) {
 // earlier writes are ordered before it, and the thread that takes the
 // count to zero sees the writes of every thread that counted down before
 // it (a fence-free completion pattern; __threadfence is a full fence).
-__device__ __forceinline__ uint32_t countdown_acq_rel(uint32_t* p) {
+__device__ __forceinline__ uint32_t add_acq_rel(uint32_t* p, uint32_t x) {
   uint32_t old;
   asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
                : "=r"(old)
-               : "l"(p), "r"(0xFFFFFFFFu)
+               : "l"(p), "r"(x)
                : "memory");
   return old;
 }
+__device__ __forceinline__ uint32_t countdown_acq_rel(uint32_t* p) { return add_acq_rel(p, 0xFFFFFFFFu); }
 
 // One atomicOr of `bit` into *word per CTA when any of its threads has `p`
 // (instead of one per warp).  Every thread of the CTA calls it.
