@@ -39,7 +39,8 @@ struct BfsWs {
   uint32_t* cursor;            // [3]
   uint32_t* hcursor;           // [3]
   int* overflow;
-  unsigned long long* stats;   // [0] arcs inspected, [1] levels, [2] unvisited arcs, [3] frontier arcs
+  unsigned long long* stats;   // [0] arcs inspected, [1] levels; [2] vertices and [3] arcs below a level
+                               // the tail hands back, [7] kInf - that level; [4..6] frontier arcs by slot
   uint32_t* mode;              // [3] 0 = top-down, 1 = bottom-up, per level slot
   uint32_t qcap, hcap;
   int adaptive;                // kBfs* schedule below
@@ -377,7 +378,13 @@ __device__ __forceinline__ void bfs_bottom_up(const GraphView& G, const BfsWs& w
 // first and lowered later; the vertices reached at the bucket's last level
 // and those a CTA could not keep go to the next superstep's queue, once each
 // (their `queued` bit).  A queue too large for narrow supersteps, or with
-// heavy vertices, is relaxed one hop by the whole grid.
+// heavy vertices, is relaxed one hop by the whole grid; from twice that size,
+// or a chunk per CTA, on the traversal goes back to its levels, whose queue,
+// direction choice and batches are made for wide frontiers (tail_back).
+// Without the way back a graph behind a chain of 20 vertices was pushed
+// through to its end: R-MAT-22, learned 2.23 -> 0.39 ms (0.42 with no tail at
+// all); eight random arcs per vertex, 4 M vertices 1.23 -> 0.75 (0.73); a grid
+// of 256^3 11.7 -> 7.4 (10.8).
 // 4096^2 grid: from the corner (8,191 levels) 48.3 -> 12.2 ms, from the
 // middle 31.6 -> 6.4; 2530 x 40 13.7 -> 2.8; 64^2 0.66 -> 0.15.  What is left
 // is 1.5 us a level, a hop's two round trips.
@@ -386,17 +393,108 @@ constexpr uint32_t kTailLevels = 64;
 using BfsDrain = DrainMem<448, 176>;
 static_assert(sizeof(BfsDrain) <= kStageWords * 4, "the slots take the staging buffers' place");
 
+// Narrow levels before the tail may take over again after it has handed back
+// (two more barriers and a pass over the labels).
+constexpr int32_t kTailPause = 64;
+
+// What bfs_tail returns beside the level at which the levels go on.
+constexpr uint32_t kTailDone = 0xFFFFFFFFu, kTailFailed = 0xFFFFFFFEu;
+
+// The least label in a queue of n light entries and nch chunks.
+__device__ __forceinline__ void back_least(const uint32_t* q, const uint4* hc, const uint32_t* dist, uint32_t n,
+                                        uint32_t nch, uint32_t gthread, uint32_t nthreads,
+                                        unsigned long long* least) {
+  uint32_t m = kInf;
+  for (uint32_t i = gthread; i < n; i += nthreads) m = min(m, ld_cg(&dist[ld_cg(&q[i])]));
+  for (uint32_t i = gthread; i < nch; i += nthreads) m = min(m, ld_cg(&dist[ld_cg(&hc[i]).x]));
+  m = __reduce_min_sync(kFull, m);
+  if (lane_id() == 0 && m < kInf) atomicMax(least, (unsigned long long)(kInf - m));
+}
+
+// Level m's frontier from the labels, which end at m from here on; the arcs
+// of the vertices in [first, m).
+__device__ __forceinline__ unsigned long long back_frontier(const GraphView& G, const BfsWs& ws, uint32_t gwarp, uint32_t nwarps,
+                                                         uint32_t m, uint32_t first) {
+  const int lane = lane_id();
+  const Frontier out{pick(ws.q, m), pick(ws.hc, m), &ws.qcount[m % 3], &ws.hcount[m % 3],
+                     ws.qcap, ws.hcap, ws.overflow};
+  WarpStage qs = frontier_stage(out, 0);
+  unsigned long long below_v = 0, below_a = 0, at_a = 0, arcs = 0;
+  for (uint32_t base = gwarp * 32; base < G.V; base += nwarps * 32) {
+    const uint32_t v = base + lane;
+    const uint32_t d = v < G.V ? ld_cg(&ws.dist[v]) : kInf;
+    if (d <= m) {
+      const uint32_t deg = __ldg(&G.row[v + 1]) - __ldg(&G.row[v]);
+      if (d == m) {
+        at_a += deg;
+      } else {
+        ++below_v;
+        below_a += deg;
+        if (d >= first) arcs += deg;
+      }
+    } else if (d < kInf) {
+      ws.dist[v] = kInf;
+    }
+    frontier_push_staged(G, out, qs, d == m, v);
+  }
+  qs.flush();
+  below_v = warp_add_u64(below_v);
+  below_a = warp_add_u64(below_a);
+  at_a = warp_add_u64(at_a);
+  if (lane == 0) {
+    if (below_v) atomicAdd(&ws.stats[2], below_v);
+    if (below_a) atomicAdd(&ws.stats[3], below_a);
+    if (at_a) atomicAdd(&ws.stats[4 + m % 3], at_a);
+  }
+  return arcs;
+}
+
+// Superstep S's queue (n light entries, nch chunks) handed back to the levels:
+// with m the least label in it, labels up to m are final.  The vertices at m
+// become level m's frontier, all of them, and what is labelled beyond m is
+// unvisited again; the counters are as the level loop leaves them, with the
+// arcs of that frontier and what lies below it (stats) for the schedules.
+// The barrier that level m starts from is the caller's.
 template <class Sync>
-__device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
-                                      unsigned long long& arcs_out) {
-  const Warps W = warps_of(s.id(), s.P());
+__device__ __forceinline__ uint32_t tail_back(Sync& s, const GraphView& G, const BfsWs& ws, const Warps& W,
+                                              uint32_t S, uint32_t n, uint32_t nch, uint32_t first,
+                                              unsigned long long& arcs_out) {
   const bool leader = s.id() == 0 && threadIdx.x == 0;
+  back_least(pick(ws.q, S), pick(ws.hc, S), ws.dist, n, nch, W.gthread, W.nthreads, &ws.stats[7]);
+  if (!s.sync()) return kTailFailed;
+  const uint32_t m =
+      kInf - (uint32_t)cta_words<1>([&](unsigned long long* w) { w[0] = ld_cg_u64(&ws.stats[7]); })[0];
+  if (leader) {  // everyone has read slot S's counts
+    for (int i = 0; i < 3; ++i) {
+      ws.qcount[i] = 0;
+      ws.hcount[i] = 0;
+      ws.cursor[i] = 0;
+      ws.hcursor[i] = 0;
+      ws.stats[4 + i] = 0;
+    }
+    ws.stats[2] = ws.stats[3] = 0;
+  }
+  if (!s.sync()) return kTailFailed;
+  if (leader) ws.stats[7] = 0;
+  arcs_out += back_frontier(G, ws, W.gwarp, W.nwarps, m, first);
+  return m;
+}
+
+template <class Sync>
+__device__ __forceinline__ uint32_t bfs_tail(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
+                                             unsigned long long& arcs_out) {
+  // the grid's shape is worked out where it is used: live across the hops it
+  // costs them 2.5 % (spills)
+  auto warps = [&] { return warps_of(s.id(), s.P()); };
   const int lane = lane_id();
   BfsDrain& m = *reinterpret_cast<BfsDrain*>(stage_mem());
   const uint32_t first = bound;
   unsigned long long walked = 0;
-  for (uint32_t i = W.gthread; i < 2 * ws.fwords; i += W.nthreads) ws.queued[i] = 0;
-  if (!s.sync()) return false;
+  {
+    const Warps W = warps();
+    for (uint32_t i = W.gthread; i < 2 * ws.fwords; i += W.nthreads) ws.queued[i] = 0;
+  }
+  if (!s.sync()) return kTailFailed;
   for (;; ++S) {
     const int cur = S % 3, nxt = (S + 1) % 3, old = (S + 2) % 3;
     const unsigned long long* sc = cta_words<2>([&](unsigned long long* w) {
@@ -405,7 +503,10 @@ __device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsW
     });
     const uint32_t n = (uint32_t)sc[0], nch = (uint32_t)sc[1];
     if (n == 0 && nch == 0) break;
-    if (leader) {
+    const unsigned long long fit = (unsigned long long)s.P() * ws.share;
+    const bool wide = nch != 0 || n > fit;
+    if (n > 2 * fit || nch > (uint32_t)s.P()) return tail_back(s, G, ws, warps(), S, n, nch, first, arcs_out);
+    if (s.id() == 0 && threadIdx.x == 0) {
       ws.qcount[old] = 0;
       ws.hcount[old] = 0;
       ws.cursor[old] = 0;
@@ -423,7 +524,7 @@ __device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsW
       atomicAnd(&in_bits[v >> 5], ~(1u << (v & 31)));
       return ld_cg(&ws.dist[v]);
     };
-    if (nch == 0 && n <= (unsigned long long)s.P() * ws.share) {
+    if (!wide) {
       drain_reset(m);
       drain_take(G, m, pick(ws.q, S), n, s.id(), s.P(), taken, push);
       uint32_t fmin = 0;
@@ -444,6 +545,7 @@ __device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsW
       };
       const uint32_t* q = pick(ws.q, S);
       const uint4* hc = pick(ws.hc, S);
+      const Warps W = warps();
       const uint32_t k = group_width(n, W.nwarps);
       WorkTaker lt((n + k - 1) / k, W, &ws.cursor[cur]);
       for (uint32_t g = lt.take(); g < lt.n; g = lt.take()) {
@@ -466,11 +568,12 @@ __device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsW
       }
       bound += 1;
     }
-    if (!s.sync()) return false;
+    if (!s.sync()) return kTailFailed;
   }
   // levels of the traversal: one more than the largest; and the arcs of the
   // vertices expanded here, each once (a vertex lowered after its expansion
   // is walked again: seven arcs in 239,000 on a 300 x 200 grid)
+  const Warps W = warps();
   uint32_t top = 0;
   for (uint32_t v = W.gthread; v < G.V; v += W.nthreads) {
     const uint32_t d = ld_cg(&ws.dist[v]);
@@ -480,12 +583,12 @@ __device__ __forceinline__ bool bfs_tail(Sync& s, const GraphView& G, const BfsW
   }
   top = __reduce_max_sync(kFull, top);
   if (lane == 0) atomicMax(&ws.stats[1], (unsigned long long)top);
-  return true;
+  return kTailDone;
 }
 
 // bfs_tail out of line, where its registers must not weigh on the levels'.
 template <class Sync>
-__device__ __noinline__ bool bfs_tail_call(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
+__device__ __noinline__ uint32_t bfs_tail_call(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
                                            unsigned long long& arcs_out) {
   return bfs_tail(s, G, ws, S, bound, arcs_out);
 }
@@ -497,8 +600,8 @@ enum { kTailNone = 0, kTailCall = 1, kTailInline = 2 };
 template <bool Hooked, int Tail, class Sync>
 __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t src,
                                          float* smlp, DecideState* dst, uint32_t* sbits) {
-  const Warps W = warps_of(s.id(), s.P());
-  const bool leader = s.id() == 0 && threadIdx.x == 0;
+  Warps W = warps_of(s.id(), s.P());
+  bool leader = s.id() == 0 && threadIdx.x == 0;
   constexpr bool hooked = Hooked;
   if constexpr (Hooked) {
     if (ws.adaptive == kBfsLearned)
@@ -539,7 +642,9 @@ __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsW
   unsigned long long arcs = 0;
   uint32_t L = 0;
   bool bottom_up = false, prev_bottom_up = false;
-  uint32_t small = 0;  // levels in a row with a small frontier
+  // levels in a row with a small frontier; negative for a while after the
+  // tail has handed back
+  int32_t small = 0;
   bool tail = false;
   // direction-choice inputs, identical in every CTA: arcs of the frontier
   // (mf) and of the still-unvisited vertices (mu).  acc[k % 3] (stats[4..6])
@@ -553,15 +658,45 @@ __device__ __forceinline__ void bfs_body(Sync& s, const GraphView& G, const BfsW
     const unsigned long long hp = sc[1];
     if (n == 0 && hp == 0) break;
     if constexpr (Tail != kTailNone) {
-      small = hp == 0 && n <= (unsigned long long)s.P() * ws.share ? small + 1 : 0;
-      if (ws.queued && small >= ws.patience) {
+      small = hp == 0 && n <= (unsigned long long)s.P() * ws.share ? small + 1 : min(small, 0);
+      if (ws.queued && small >= (int32_t)ws.patience) {
         // the tail reads slot L's counts again; the slot after next is its to clear
-        bool done;
-        if constexpr (Tail == kTailCall) done = bfs_tail_call(s, G, ws, L, L, arcs);
-        else done = bfs_tail(s, G, ws, L, L, arcs);
-        if (!done) return;
-        tail = true;
-        break;
+        uint32_t back;
+        if constexpr (Tail == kTailCall) back = bfs_tail_call(s, G, ws, L, L, arcs);
+        else back = bfs_tail(s, G, ws, L, L, arcs);
+        if (back == kTailFailed) return;
+        if (back == kTailDone) {
+          tail = true;
+          break;
+        }
+        L = back;
+        if constexpr (Hooked) {
+          if (!s.sync_hook([&] {
+                if (threadIdx.x == 0) {
+                  dst->vis_v = ld_cg_u64(&ws.stats[2]);
+                  dst->vis_a = ld_cg_u64(&ws.stats[3]);
+                }
+                __syncthreads();
+                bfs_decide(G, ws, smlp, dst, L, W.nwarps);
+              }))
+            return;
+        } else {
+          if (!s.sync()) return;
+          // as the loop leaves them before level L (nothing of the old
+          // ones is live across the tail)
+          const unsigned long long* w = cta_words<2>([&](unsigned long long* x) {
+            x[0] = ld_cg_u64(&ws.stats[3]);
+            x[1] = ld_cg_u64(&ws.stats[4 + L % 3]);
+          });
+          mf = w[1];
+          mu = G.E - (L > 0 ? w[0] : w[1]);
+        }
+        bottom_up = prev_bottom_up = false;
+        small = -kTailPause;
+        W = warps_of(s.id(), s.P());
+        leader = s.id() == 0 && threadIdx.x == 0;
+        --L;
+        continue;
       }
     }
     if (ws.adaptive == kBfsHeuristic) {
