@@ -1008,12 +1008,24 @@ static int bfs_mode(gdb_ctx* c, const gdb_graph* g, int* mode) {
 // loop registers (R-MAT, threshold schedule, one source: 0.270 -> 0.279 ms;
 // the learned kernel's levels run no slower with it, 0.301 -> 0.292, but on
 // lanes they do, 16 sources 2.85 -> 2.89 ms).  So it is there for graphs of
-// at most 8 arcs per vertex on average -- grids, meshes, roads; R-MAT graphs
-// have 16 and more -- and for learned traversals that have the GPU to
-// themselves, batches of uneven graphs among them.
+// at most 8 arcs per vertex on average -- grids, meshes, roads; most R-MAT
+// graphs have 16 and more -- and for learned traversals that have the GPU to
+// themselves, batches of uneven graphs among them.  Not for large graphs with
+// hubs, which are wide rather than long and whose pulls want the third CTA
+// per SM.  Threshold schedule without the tail -> with it, R-MAT of edge
+// factor 2 and 4: 0.3 M vertices 0.106 -> 0.089 and 0.107 -> 0.090 ms, 1 M
+// 0.137 -> 0.128 and 0.131 -> 0.120, 2.1 M 0.172 -> 0.170 and 0.192 -> 0.192,
+// 4.2 M 0.225 -> 0.236 and 0.233 -> 0.252, 8.4 M 0.396 -> 0.472 and 0.394 ->
+// 0.455.  (Pushed only they run as fast either way: 4.2 M 0.55 -> 0.54, 8.4 M
+// 0.65 -> 0.65.)  Without hubs a large graph may be either: random graphs of 6
+// arcs per vertex lose as R-MAT does (8.4 M 0.74 -> 0.77, 16.8 M of 4 arcs
+// 1.45 -> 1.81), a 4096^2 grid with one vertex of 24 arcs wins 63.7 -> 12.0,
+// and the tail stays.
+constexpr uint32_t kHubTailV = 1u << 21;
 static const void* bfs_kernel(const gdb_graph* g, int mode, bool alone, bool tail) {
   if (mode >= kBfsLearned) return tail && alone ? (const void*)k_bfs_xf_sel_tail : (const void*)k_bfs_xf_sel;
-  return tail && g->E <= 8ull * g->V ? (const void*)k_bfs_xf_tail : (const void*)k_bfs_xf;
+  const bool hubs = g->nheavy > 0 && g->V > kHubTailV;
+  return tail && g->E <= 8ull * g->V && !hubs ? (const void*)k_bfs_xf_tail : (const void*)k_bfs_xf;
 }
 
 using BfsKernel = void (*)(gdb::DiscoveryArgs, gdb::GraphView, BfsWs, uint32_t);
