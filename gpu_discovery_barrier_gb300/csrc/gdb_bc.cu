@@ -15,8 +15,9 @@
 //  * forward, level L -> L+1, direction-optimising: push -- the level's
 //    vertices claim unvisited neighbours (CAS on d) and add their path
 //    count into every level-L+1 neighbour's (an FP32 L2 atomic, as the
-//    reference's float adds; FP64 ones cost 6 % more of the BC time); pull -- every unvisited vertex sums the path counts of its
-//    level-L neighbours and claims itself when the sum is positive.  A
+//    reference's float adds; FP64 ones cost 6 % more of the BC time); pull --
+//    every unvisited vertex sums the path counts of its level-L neighbours
+//    and claims itself when the sum is positive.  A
 //    pull has no early exit (every parent counts), so it runs when the
 //    unvisited vertices' arcs are fewer than three times the level's own (a
 //    pushed arc ends in an atomic);
@@ -86,39 +87,11 @@ struct BcWs {
   unsigned long long* stats;     // [0] arcs, [1] supersteps, [2] reached arcs (work units)
 };
 
-// Visit one level segment: light groups over order[lb, lb+nl) (begin/edge/
-// end hooks) and the level's heavy chunk entries hc[hcb, hcb+nch), whose
-// vertex slots start at hvb: heavy(v, slot, chunks_of_v, arc_begin, arc_end).
-template <class Begin, class Edge, class End, class Heavy>
-__device__ __forceinline__ void visit_level(const GraphView& G, const Warps& W, const BcWs& ws,
-                                            uint32_t lb, uint32_t nl, uint32_t hcb, uint32_t hvb,
-                                            uint32_t nch, uint32_t* cursor, uint32_t* hcursor,
-                                            Begin&& begin, Edge&& edge, End&& end, Heavy&& heavy) {
-  const int lane = lane_id();
-  const uint32_t k = group_width(nl, W.nwarps);
-  WorkTaker lt((nl + k - 1) / k, W, cursor);
-  for (uint32_t g = lt.take(); g < lt.n; g = lt.take()) {
-    const uint32_t i = g * k + lane;
-    const bool act = (uint32_t)lane < k && i < nl;
-    const uint32_t v = act ? ld_cg(&ws.order[lb + i]) : 0u;
-    begin(v, act);
-    __syncwarp();
-    group_arcs(G, act, v, edge);
-    __syncwarp();
-    end(v, act);
-  }
-  WorkTaker ht(nch, W, hcursor, lt.n);
-  for (uint32_t c = ht.take(); c < nch; c = ht.take()) {
-    const uint4 ent = ld_cg(&ws.hc[hcb + c]);
-    uint32_t b, en;
-    chunk_range(G, ent, b, en);
-    heavy(ent.x, hvb + ent.z, ent.w, b, en);
-  }
-}
-
-// visit_level with four 32-arc steps per call of edge4(valid[4], owner[4],
-// arc[4]) (group_arcs4): a step's dependent loads are in flight together
-// with the next three steps'.
+// Visit one level segment: light groups over order[lb, lb+nl) (begin and end
+// hooks; edge4(valid[4], owner[4], arc[4]) per four 32-arc steps, group_arcs4,
+// whose dependent loads are in flight together) and the level's heavy chunk
+// entries hc[hcb, hcb+nch), whose vertex slots start at hvb: heavy(v, slot,
+// chunks_of_v, arc_begin, arc_end).
 template <class Begin, class Edge4, class End, class Heavy>
 __device__ __forceinline__ void visit_level4(const GraphView& G, const Warps& W, const BcWs& ws,
                                              uint32_t lb, uint32_t nl, uint32_t hcb, uint32_t hvb,
@@ -167,13 +140,6 @@ __device__ __forceinline__ float four_sums(const float* x) {
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(kFull, z, o);
   return z;
-}
-
-// a + b; err: what rounding took from it, exactly (Knuth's two-sum).
-__device__ __forceinline__ float two_sum(float a, float b, float& err) {
-  const float t = __fadd_rn(a, b), z = __fsub_rn(t, a);
-  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
-  return t;
 }
 
 __device__ __forceinline__ int32_t level_of(const BcWs& ws, uint32_t v) {

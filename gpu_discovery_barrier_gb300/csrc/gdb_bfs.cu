@@ -413,8 +413,8 @@ __device__ __forceinline__ void back_least(const uint32_t* q, const uint4* hc, c
 
 // Level m's frontier from the labels, which end at m from here on; the arcs
 // of the vertices in [first, m).
-__device__ __forceinline__ unsigned long long back_frontier(const GraphView& G, const BfsWs& ws, uint32_t gwarp, uint32_t nwarps,
-                                                         uint32_t m, uint32_t first) {
+__device__ __forceinline__ unsigned long long back_frontier(const GraphView& G, const BfsWs& ws, uint32_t gwarp,
+                                                           uint32_t nwarps, uint32_t m, uint32_t first) {
   const int lane = lane_id();
   const Frontier out{pick(ws.q, m), pick(ws.hc, m), &ws.qcount[m % 3], &ws.hcount[m % 3],
                      ws.qcap, ws.hcap, ws.overflow};
@@ -481,8 +481,8 @@ __device__ __forceinline__ uint32_t tail_back(Sync& s, const GraphView& G, const
 }
 
 template <class Sync>
-__device__ __forceinline__ uint32_t bfs_tail(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
-                                             unsigned long long& arcs_out) {
+__device__ __forceinline__ uint32_t bfs_tail(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S,
+                                             uint32_t bound, unsigned long long& arcs_out) {
   // the grid's shape is worked out where it is used: live across the hops it
   // costs them 2.5 % (spills)
   auto warps = [&] { return warps_of(s.id(), s.P()); };
@@ -588,8 +588,8 @@ __device__ __forceinline__ uint32_t bfs_tail(Sync& s, const GraphView& G, const 
 
 // bfs_tail out of line, where its registers must not weigh on the levels'.
 template <class Sync>
-__device__ __noinline__ uint32_t bfs_tail_call(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S, uint32_t bound,
-                                           unsigned long long& arcs_out) {
+__device__ __noinline__ uint32_t bfs_tail_call(Sync& s, const GraphView& G, const BfsWs& ws, uint32_t S,
+                                               uint32_t bound, unsigned long long& arcs_out) {
   return bfs_tail(s, G, ws, S, bound, arcs_out);
 }
 
@@ -970,9 +970,8 @@ static void bfs_bitmap(gdb_ctx* c, const gdb_graph* g, BfsWs* ws, bool alone, si
 
 int gdbi::bfs_prepare(gdb_ctx* c) {
   // static + dynamic shared memory above 48 KB needs each kernel's opt-in
-  for (const void* k : {(const void*)k_bfs_xf, (const void*)k_bfs_xf_tail, (const void*)k_bfs_xf_sel, (const void*)k_bfs_xf_sel_tail,
-                        (const void*)k_bfs_grid,
-                        (const void*)k_bfs_grid_sel})
+  for (const void* k : {(const void*)k_bfs_xf, (const void*)k_bfs_xf_tail, (const void*)k_bfs_xf_sel,
+                        (const void*)k_bfs_xf_sel_tail, (const void*)k_bfs_grid, (const void*)k_bfs_grid_sel})
     GDB_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageKbMax * 1024));
   return GDB_OK;
 }

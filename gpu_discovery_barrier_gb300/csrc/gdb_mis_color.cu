@@ -5,10 +5,11 @@
 // undecided neighbours (mis1, :245-270); undecided strict local minima join
 // the set, s = 2, and mark their undecided neighbours decided (mis2,
 // :277-312).  What decides is whether some undecided neighbour is at or
-// below the vertex's own priority, so a vertex here stops at the first.  The reference stages neighbour marks in cu[] and commits them
-// in a third barrier interval (mis3, :322-330); here the marks go straight
-// into the state array -- two winners are never adjacent, so no winner test
-// can see a mark of the same round -- and a round needs two barriers.
+// below the vertex's own priority, so a vertex here stops at the first.  The
+// reference stages neighbour marks in cu[] and commits them in a third barrier
+// interval (mis3, :322-330); here the marks go straight into the state array
+// -- two winners are never adjacent, so no winner test can see a mark of the
+// same round -- and a round needs two barriers.
 //
 // Colouring (mega_kernel, pannotia/graph_app/color/kernel/color_kernel.cl:159-252):
 // per round every uncoloured vertex takes the maximum priority over its

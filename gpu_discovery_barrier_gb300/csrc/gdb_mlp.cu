@@ -16,6 +16,7 @@
 
 #include "gdb_internal.h"
 #include "gdb_selector.cuh"
+#include "gdb_sweep.cuh"
 
 using namespace gdbi;
 using namespace gdb;
@@ -83,13 +84,6 @@ constexpr int kRXn = 0, kRH1 = kRXn + kFeat, kRH2 = kRH1 + kH1, kRDh1 = kRH2 + k
 constexpr int kMlpThreads = 256;
 constexpr int kMlpSmem = (kRows * kPitch + ((kRows + 3) & ~3) + ((kParams + 3) & ~3)) * 4;
 static_assert(kPW1 % 4 == 0 && kPW2 % 4 == 0, "weight rows are read as float4");
-
-// a + b; err: what rounding took from it, exactly.
-__device__ __forceinline__ float two_sum(float a, float b, float& err) {
-  const float t = __fadd_rn(a, b), z = __fsub_rn(t, a);
-  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
-  return t;
-}
 
 // Largest magnitude of a product or column value that a run of floats takes
 // (2^32 values on 304 CTAs stay below 1e36), and the tiles of
@@ -176,8 +170,9 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
   auto entry = [&](int i, int j) { return out0 - kPW1 + i * outw + j * ocol; };
   // column c's entry: dh1, dh2 and dy are the biases; the loss is the last one
   auto column = [&](int c) {
-    return (c < kH1 ? kPB1 + c : c < kH1 + kH2 ? kPB2 + c - kH1 : c < kH1 + kH2 + kOut ? kPB3 + c - kH1 - kH2 : kParams) -
-           kPW1;
+    const int e = c < kH1 ? kPB1 + c : c < kH1 + kH2 ? kPB2 + c - kH1
+                : c < kH1 + kH2 + kOut ? kPB3 + c - kH1 - kH2 : kParams;
+    return e - kPW1;
   };
   auto end_run = [&] {
 #pragma unroll

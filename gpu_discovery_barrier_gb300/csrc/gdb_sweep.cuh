@@ -82,15 +82,11 @@ __device__ __forceinline__ T pick(const T (&a)[2], uint32_t i) {
   return (i & 1) ? a[1] : a[0];
 }
 
-// Order-preserving float <-> uint32 map (so atomicMin/Max on uint32 order
+// Order-preserving float -> uint32 map (so atomicMin/Max on uint32 order
 // floats; -0 is folded onto +0 first).
 __device__ __forceinline__ uint32_t fkey(float f) {
   uint32_t b = __float_as_uint(f == 0.0f ? 0.0f : f);
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float fkey_inv(uint32_t k) {
-  uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-  return __uint_as_float(b);
 }
 
 // Warp identity among the participating CTAs.
@@ -580,31 +576,9 @@ __device__ __forceinline__ void for_groups(uint32_t ngroups, const Warps& W, uin
 
 // Sweep the light vertices of [0, V) in warp groups of 32 consecutive ids.
 // begin(v, in_range) -> bool active: per-lane setup (v is light and < V
-// when in_range); edge(valid, owner_lane, arc) per 32-arc step;
+// when in_range); edge4(valid[4], owner_lane[4], arc[4]) per four 32-arc
+// steps (group_arcs4), whose dependent loads are in flight together;
 // end(v, active) after the group's arcs.  Groups come from `cursor`.
-template <class Begin, class Edge, class End>
-__device__ __forceinline__ void sweep_light(const GraphView& G, uint32_t* cursor, Begin&& begin,
-                                            Edge&& edge, End&& end) {
-  const int lane = lane_id();
-  const uint32_t ngroups = (G.V + 31) / 32;
-  for (;;) {
-    const uint32_t g0 = warp_grab(cursor) * kGrab;
-    if (g0 >= ngroups) break;
-    for (uint32_t g = g0; g < min(g0 + kGrab, ngroups); ++g) {
-      const uint32_t v = g * 32 + lane;
-      const bool in_range = v < G.V && !is_heavy(G, v);
-      const bool act = begin(v, in_range) && in_range;
-      __syncwarp();
-      group_arcs(G, act, v, edge);
-      __syncwarp();
-      end(v, act);
-    }
-  }
-}
-
-// sweep_light with four 32-arc steps per call of edge4(valid[4],
-// owner_lane[4], arc[4]) (group_arcs4), so a step's dependent loads are in
-// flight together with the next three steps'.
 template <class Begin, class Edge4, class End>
 __device__ __forceinline__ void sweep_light4(const GraphView& G, uint32_t* cursor, Begin&& begin,
                                              Edge4&& edge4, End&& end) {
@@ -627,10 +601,9 @@ __device__ __forceinline__ void sweep_light4(const GraphView& G, uint32_t* curso
 }
 
 // Sweep the heavy vertices through the static chunk table, kGrab chunks
-// per grab: fn(chunk, v, heavy_index, chunk_in_vertex, arc_begin, arc_end),
-// chunk = the entry's index in the table.
+// per grab: fn(v, heavy_index, chunk_in_vertex, arc_begin, arc_end).
 template <class Fn>
-__device__ __forceinline__ void sweep_heavy_indexed(const GraphView& G, uint32_t* hcursor, Fn&& fn) {
+__device__ __forceinline__ void sweep_heavy(const GraphView& G, uint32_t* hcursor, Fn&& fn) {
   for (;;) {
     const uint32_t c0 = warp_grab(hcursor) * kGrab;
     if (c0 >= G.nheavy_chunks) break;
@@ -638,24 +611,12 @@ __device__ __forceinline__ void sweep_heavy_indexed(const GraphView& G, uint32_t
       const uint4 ent = __ldg(&G.heavy_chunk[c]);
       uint32_t b, en;
       chunk_range(G, ent, b, en);
-      fn(c, ent.x, ent.z, ent.y, b, en);
+      fn(ent.x, ent.z, ent.y, b, en);
     }
   }
 }
 
-// sweep_heavy_indexed without the chunk index:
-// fn(v, heavy_index, chunk_in_vertex, arc_begin, arc_end).
-template <class Fn>
-__device__ __forceinline__ void sweep_heavy(const GraphView& G, uint32_t* hcursor, Fn&& fn) {
-  sweep_heavy_indexed(G, hcursor, [&](uint32_t, uint32_t v, uint32_t h, uint32_t j, uint32_t b, uint32_t e) {
-    fn(v, h, j, b, e);
-  });
-}
-
 // Warp reductions.
-__device__ __forceinline__ uint32_t warp_min_u32(uint32_t x) { return __reduce_min_sync(kFull, x); }
-__device__ __forceinline__ uint32_t warp_max_u32(uint32_t x) { return __reduce_max_sync(kFull, x); }
-__device__ __forceinline__ uint32_t warp_or_u32(uint32_t x) { return __reduce_or_sync(kFull, x); }
 __device__ __forceinline__ uint32_t warp_add_u32(uint32_t x) { return __reduce_add_sync(kFull, x); }
 __device__ __forceinline__ unsigned long long warp_add_u64(unsigned long long x) {
 #pragma unroll
@@ -729,6 +690,13 @@ __device__ __forceinline__ void segment_add(double* slot, int owner, float x) {
     if (o <= rest) x += y;
   }
   if (head && __float_as_uint(x) != 0x80000000u) slot[owner] += (double)x;
+}
+
+// a + b; err: what rounding took from it, exactly (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float t = __fadd_rn(a, b), z = __fsub_rn(t, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
+  return t;
 }
 
 __device__ __forceinline__ float warp_sum_f32(float x) {
