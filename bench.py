@@ -128,13 +128,14 @@ def reach(g, dist):
 
 # -------------------------------------------------------------- roofline
 
-def alg_bytes(app: str, g, reached, rounds: int) -> float:
-    """Algorithmic bytes of one launch (uint32 = 4 B), schedule-independent:
+def alg_bytes(app: str, g, reached, rounds: int, arcs: int = 0) -> float:
+    """Algorithmic bytes of one launch (uint32 = 4 B):
     BFS 8E_r + 12V_r + 4V; SSSP 12E_r + 12V_r + 4V; BC 20E_r + 24V_r + 12V
     per source; MST (12E + 16V) per round; colouring 24E + 16V (one count
-    pass and one countdown pass over the arcs); MIS 4E once, bounded from
-    above by the full graph (a vertex stops at the first neighbour that beats
-    it), and 8V per round."""
+    pass and one countdown pass over the arcs); MIS 8 per arc the kernel
+    inspected (`arcs`: column and key; a vertex stops at the first neighbour
+    that beats it) and 12V (priority, key, result).  All but MIS's follow
+    from the graph and the result alone."""
     V, E = g.V, g.E
     if app == "bfs":
         return sum(8 * er + 12 * vr + 4 * V for vr, er in reached)
@@ -148,7 +149,7 @@ def alg_bytes(app: str, g, reached, rounds: int) -> float:
         # count pass (col + neighbour priority per arc) and one countdown
         # pass (col, neighbour degree and priority, counter) per arc
         return 8 * E + 8 * V + 16 * E + 8 * V
-    return 4 * E + rounds * 8 * V
+    return 8 * arcs + 12 * V
 
 
 def peaks():
@@ -264,11 +265,12 @@ class GpuSuite:
 
         def note(app):
             st = c.last_stats()
-            r = record.setdefault(app, {"ms": 0.0, "launches": 0, "calls": 0, "supersteps": 0})
+            r = record.setdefault(app, {"ms": 0.0, "launches": 0, "calls": 0, "supersteps": 0, "arcs": 0})
             r["ms"] += st["kernel_ms"]
             r["launches"] += st["launches"]
             r["calls"] += 1
             r["supersteps"] += st["supersteps"]
+            r["arcs"] += st["edges_processed"]
 
         # the 16 sources' independent runs, spread over concurrent lanes
         if "bfs" in self.apps:
@@ -724,7 +726,7 @@ def run_gdb(args, rank, world, local):
         if app in ("bfs", "sssp", "bc"):
             nbytes = alg_bytes(app, g, reached, 0)
         else:
-            nbytes = alg_bytes(app, g, [], rounds)
+            nbytes = alg_bytes(app, g, [], rounds, r["arcs"] // r["calls"])
         return nbytes, launch_ms, nbytes / (launch_ms / 1e3) / 1e9
 
     per_app_roof = {a: round(app_roofline(a)[2] / peak, 4) for a in rec}
