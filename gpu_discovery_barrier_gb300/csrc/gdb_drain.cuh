@@ -40,7 +40,10 @@ template <uint32_t Cap, uint32_t List>
 struct DrainMem {
   static constexpr uint32_t kCap = Cap;   // arc slots per buffer
   static constexpr uint32_t kList = List;
-  static constexpr uint32_t kPile = Cap / 2;  // pile entries per CTA up to which a phase change is narrow
+  // pile entries per CTA up to which a phase change is narrow (Cap / 4, / 2 and
+  // Cap itself are the same on grids of 4,096 to 16.8 M vertices and in mixed
+  // batches, within 0.4 %)
+  static constexpr uint32_t kPile = Cap / 2;
   uint32_t arc[2][Cap], v[2][Cap], d[2][Cap];
   uint32_t far[List];    // reached at or beyond the bucket's end
   uint32_t spill[List];  // handed to the next superstep's frontier

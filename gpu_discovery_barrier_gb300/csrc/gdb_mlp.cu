@@ -585,7 +585,8 @@ void gdbi::sssp_features(gdb_ctx* c, const gdb_graph* g, uint32_t nsrc, float* x
   const double V = g->V, E = (double)g->E;
   const double nf = std::min<double>(nsrc, V);
   const double mf = nf * E / std::max(V, 1.0);
-  // warps of the launch: the traversal kernels' resident CTAs, capped by max_ctas
+  // warps of the launch as the network was trained: the traversal kernels'
+  // resident CTAs, capped by max_ctas (small_shape's cut is not in the traces)
   double ctas = (double)c->sm_count * std::max(gdbi::traversal_occupancy(c, c->opt.block_size), 1);
   if (c->opt.max_ctas > 0) ctas = std::min(ctas, (double)c->opt.max_ctas);
   const double warps = ctas * (c->opt.block_size / 32);

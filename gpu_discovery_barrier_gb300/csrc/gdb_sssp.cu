@@ -1085,7 +1085,11 @@ static size_t sssp_layout(const gdb_graph* g, char* base, uint32_t* d_dist, Sssp
   ws->trace_cap = 0;
   ws->maxdeg = g->maxdeg;
   ws->share = drain_share(g->E, V, SsspDrain::kCap);
-  // a graph of at most 8 arcs per vertex has no wide supersteps to wait for
+  // a graph of at most 8 arcs per vertex rarely has wide supersteps to wait
+  // for.  The first number hardly matters (1 / 2 / 4: 4096^2 grid, BFS and SSSP
+  // 33.2 / 33.1 / 33.1 ms, a grid of 50,000 1.22 / 1.23 / 1.17), nor the second
+  // (1 / 2 / 4 / 8: 64 mixed graphs 12.35 / 12.35 / 12.36 / 12.36, 16 of up to
+  // 30,000 6.82 / 6.82 / 6.72 / 6.82)
   ws->patience = g->maxdeg <= 8 ? 1u : 4u;
   ws->light = kInf;
   ws->qcap = V;
@@ -1143,9 +1147,10 @@ static int sssp_auto_delta(gdb_ctx* c, gdb_graph* g, uint32_t* delta) {
 // U[1,255] weights (the rule's width 134), 16 sources on lanes:
 //   width 24: 16.4 ms, 28: 15.4, 32: 15.6, 40: 17.3, 48: 18.2, 67: 20.6,
 //   96: 25.3, 134: 31.9 ms.
-// Graphs whose weights stay below half the width (the 4096^2 grid: width
-// 1,024, no split) keep the full width, where narrower buckets only add
-// supersteps (grid SSSP 108 ms at 1,024, 131 at 512, 157 at 256).
+// Graphs whose weights stay below half the width (the 4096^2 grid with
+// weights to 255: width 1,024, no split) keep the full width, where narrower
+// buckets only add supersteps (grid SSSP 30.4 ms at 512, 24.4 at 1,024, 21.0 at
+// 2,048 and 4,096, 25.8 at 8,192).
 static int sssp_auto_width(gdb_ctx* c, gdb_graph* g, uint32_t* delta) {
   int rc = sssp_auto_delta(c, g, delta);
   if (rc || c->opt.sssp_split < 0 || *delta < 2) return rc;
@@ -1235,6 +1240,11 @@ static int settle_of(const gdb_ctx* c, uint32_t light, int force) {
 // The XF kernel of a run.  Narrow supersteps need whole arcs (no split) and
 // pay where frontiers are small for long: near-far runs, graphs of at most 8
 // arcs per vertex on average, and graphs whose every frontier is small.
+// Wide graphs that it takes too lose nothing by it, k_sssp_xf -> narrow:
+// near-far without the split on R-MAT of 16 arcs per vertex, 65,536 vertices
+// 0.295 -> 0.267 ms, 1 M 1.33 -> 1.30, 4.2 M 3.97 -> 3.98; worklist on R-MAT of
+// edge factor 2 and 4, 1 M 0.54 -> 0.52 and 0.65 -> 0.63, 8.4 M 2.26 -> 2.26 and
+// 3.41 -> 3.40.
 // What is left to k_sssp_xf besides the split is the plain worklist on
 // R-MAT-like graphs, a dozen wide supersteps that the narrow kernel's shared
 // memory slows (R-MAT-22 3.93 -> 4.0 to 4.1 ms per source), and the plain
