@@ -2,7 +2,7 @@
 //
 // Training is full-batch Adam over a masked squared loss.  One step is two
 // kernels:
-//   k_mlp_grad  a CTA takes tiles of 128 samples: forward and backward pass
+//   k_mlp_grad  a CTA takes tiles of up to 128 samples: forward and backward pass
 //               into shared memory, then the tile's share of every gradient
 //               entry from there (register tiles of 4 x 4 entries), kept in
 //               FP64 registers from tile to tile;
@@ -114,7 +114,7 @@ constexpr uint32_t kRunTiles = 8;
 // 135,000 samples: 1.9 -> 0.17 ms a step, k_mlp_step included.
 __global__ void __launch_bounds__(kMlpThreads, 2)
     k_mlp_grad(const float* __restrict__ p, const float* __restrict__ X, const float* __restrict__ T,
-               const float* __restrict__ M, uint32_t n, const float* __restrict__ inv_mask,
+               const float* __restrict__ M, uint32_t n, uint32_t span, const float* __restrict__ inv_mask,
                double* __restrict__ part) {
   extern __shared__ float4 mlp_smem[];
   float* act = reinterpret_cast<float*>(mlp_smem);  // [kRows][kPitch]
@@ -187,9 +187,10 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
   };
   uint32_t run = 0;
 
-  for (uint32_t tile = blockIdx.x; (size_t)tile * kTile < n; tile += gridDim.x) {
-    const size_t base = (size_t)tile * kTile;
-    const uint32_t have = n - base < (size_t)kTile ? (uint32_t)(n - base) : (uint32_t)kTile;
+  const int halfspan = (int)span / 2;
+  for (uint32_t tile = blockIdx.x; (size_t)tile * span < n; tile += gridDim.x) {
+    const size_t base = (size_t)tile * span;
+    const uint32_t have = n - base < (size_t)span ? (uint32_t)(n - base) : span;
     // targets and masks of thread tid < 128's sample, in flight early
     float tt[kOut], mm[kOut];
     if (tid < kTile) {
@@ -322,11 +323,11 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) fits = fits && top[a0 + i * as] * top[d0 + drow(j)] < kRunMax;
-      const float* A = act + a0 * kPitch + 64 * half;
-      const float* D = act + d0 * kPitch + 64 * half;
+      const float* A = act + a0 * kPitch + halfspan * half;
+      const float* D = act + d0 * kPitch + halfspan * half;
       if (fits) {
 #pragma unroll 1
-        for (int s = 0; s < 64; s += 4) {
+        for (int s = 0; s < halfspan; s += 4) {
           float av[4][4], dv[4][4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
             const float *x = A + i * as * kPitch, *y = D + drow(j) * kPitch;
             double t = 0.0;
 #pragma unroll 1
-            for (int s = 0; s < 64 && 64 * half + s < (int)have; ++s) t += (double)x[s] * (double)y[s];
+            for (int s = 0; s < halfspan && halfspan * half + s < (int)have; ++s) t += (double)x[s] * (double)y[s];
             if (j < nd) put(entry(i, j), t);
           }
         begun = true;
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
       const float* c0 = act + (kRDh1 + colr0) * kPitch;
       const float* c1 = act + (kRDh1 + (colr1 < kCols ? colr1 : colr0)) * kPitch;
 #pragma unroll 4
-      for (int s = 0; s < kTile; ++s)
+      for (uint32_t s = 0; s < span; ++s)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           float e0, e1;
@@ -440,6 +441,7 @@ struct MlpBufs {
   double *loss = nullptr, *part = nullptr;
   char* base = nullptr;
   int ctas = 0;
+  uint32_t span = kTile;  // samples of a CTA's tile
 };
 
 // 1 / sum of the mask (0 for an empty one).
@@ -451,8 +453,16 @@ __global__ void k_mask_inverse(const double* __restrict__ part, float* __restric
 
 int mlp_upload(gdb_ctx* c, MlpBufs& b, const float* params, const float* x, const float* t,
                const float* m, uint32_t n, bool adam) {
-  // two CTAs per SM hold the tiles; fewer tiles take a CTA each
-  b.ctas = (int)std::min<uint64_t>(2ull * c->sm_count, ((uint64_t)n + kTile - 1) / kTile);
+  // two CTAs per SM hold the tiles; fewer tiles take a CTA each.  A step on
+  // few samples lasts as long as one tile's products, so they go in tiles of
+  // 16, 32 or 64 while these are no more than the SMs; more tiles cost more
+  // sums (20 epochs and a forward, tiles of 16 / 32 / 64 / 128: 1,000 samples
+  // 0.58 / 0.62 / 0.71 / 0.87 ms, 4,000 0.83 / 0.70 / 0.75 / 0.91, 6,000 0.95 /
+  // 0.83 / 0.75 / 0.91, 10,000 1.16 / 1.00 / 0.89 / 0.92, 20,000 1.61 / 1.30 /
+  // 1.20 / 1.19)
+  b.span = 16;
+  while (b.span < (uint32_t)kTile && (uint64_t)b.span * c->sm_count < n) b.span *= 2;
+  b.ctas = (int)std::min<uint64_t>(2ull * c->sm_count, ((uint64_t)n + b.span - 1) / b.span);
   GDB_CUDA(c, cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlpSmem));
   Bump bp;
   const size_t o_p = bp.take(kParams * 4), o_x = bp.take((size_t)n * kFeat * 4),
@@ -488,7 +498,8 @@ int mlp_upload(gdb_ctx* c, MlpBufs& b, const float* params, const float* x, cons
 
 // Gradient and loss, then the Adam update where b has its moments.
 int mlp_step(gdb_ctx* c, MlpBufs& b, uint32_t n, float lr_t, float wd) {
-  k_mlp_grad<<<b.ctas, kMlpThreads, kMlpSmem, c->stream>>>(b.p, b.x, b.t, b.m, n, b.inv_mask, b.part);
+  k_mlp_grad<<<b.ctas, kMlpThreads, kMlpSmem, c->stream>>>(b.p, b.x, b.t, b.m, n, b.span, b.inv_mask,
+                                                         b.part);
   k_mlp_step<<<(kGradEntries + 1 + 7) / 8, 256, 0, c->stream>>>(b.part, 2 * b.ctas, b.g, b.loss, b.p, b.m1,
                                                                 b.m2, lr_t, wd);
   GDB_CUDA(c, cudaGetLastError());
