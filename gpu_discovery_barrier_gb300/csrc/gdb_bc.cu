@@ -401,10 +401,11 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
     // rounded once, by the warp that brings the vertex's last chunk, which
     // also claims it.  (FP32 atomics of the chunks' sums lost what stays
     // under half a unit of a hub's count, and depended on their order.)
+    const uint32_t hk = chunk_width(G.nheavy_chunks, W.nwarps);
     while (nhvbase < G.nheavy) {  // some left
-      const uint32_t base = warp_grab(&ws.hcursor[cur]) * 32;
+      const uint32_t base = warp_grab(&ws.hcursor[cur]) * hk;
       if (base >= G.nheavy_chunks) break;
-      const uint4 ent = base + lane < G.nheavy_chunks ? __ldg(&G.heavy_chunk[base + lane]) : make_uint4(0, 0, 0, 0);
+      const uint4 ent = (uint32_t)lane < hk && base + lane < G.nheavy_chunks ? __ldg(&G.heavy_chunk[base + lane]) : make_uint4(0, 0, 0, 0);
       const bool open = ent.w && level_of(ws, ent.x) == -1;  // until its last chunk is in
       uint32_t rb = 0, re = 0;
       if (open) {

@@ -74,11 +74,11 @@ __device__ __forceinline__ void mis_init(const GraphView& G, const Warps& W, con
   }
 }
 
-// The warp's 32 chunk entries from `base`, one per lane; past the table's
-// end: no entry (w = 0 chunks).
-__device__ __forceinline__ uint4 mis_chunk(const GraphView& G, uint32_t base) {
+// The warp's k chunk entries from `base`, one per lane; the other lanes and
+// past the table's end: no entry (w = 0 chunks).
+__device__ __forceinline__ uint4 mis_chunk(const GraphView& G, uint32_t base, uint32_t k) {
   const uint32_t c = base + lane_id();
-  return c < G.nheavy_chunks ? __ldg(&G.heavy_chunk[c]) : make_uint4(0, 0, 0, 0);
+  return (uint32_t)lane_id() < k && c < G.nheavy_chunks ? __ldg(&G.heavy_chunk[c]) : make_uint4(0, 0, 0, 0);
 }
 
 // mis1 of round r: an undecided vertex with an undecided neighbour at or
@@ -161,8 +161,9 @@ __device__ __forceinline__ void mis_phase1(const GraphView& G, const Warps& W, c
   }
   win.flush();
   lose.flush();
-  for (uint32_t base = W.gwarp * 32; heavy && base < G.nheavy_chunks; base += W.nwarps * 32) {
-    const uint4 ent = mis_chunk(G, base);
+  const uint32_t k = chunk_width(G.nheavy_chunks, W.nwarps);
+  for (uint32_t base = W.gwarp * k; heavy && base < G.nheavy_chunks; base += W.nwarps * k) {
+    const uint4 ent = mis_chunk(G, base, k);
     bool todo = ent.w != 0 && ld_cg(&ws.state[ent.x]) == -1;
     if (todo && ld_cg(&ws.s[ent.x]) == 2) {
       // a heavy winner's own state is settled here (see mis2)
@@ -253,8 +254,9 @@ __device__ __forceinline__ void mis_phase2(const GraphView& G, const Warps& W, c
   // round settles its state (all its neighbours are decided by then, so
   // nobody reads it in between).
   bool any_win = false;
-  for (uint32_t base = W.gwarp * 32; heavy && base < G.nheavy_chunks; base += W.nwarps * 32) {
-    const uint4 ent = mis_chunk(G, base);
+  const uint32_t hk = chunk_width(G.nheavy_chunks, W.nwarps);
+  for (uint32_t base = W.gwarp * hk; heavy && base < G.nheavy_chunks; base += W.nwarps * hk) {
+    const uint4 ent = mis_chunk(G, base, hk);
     const bool won = ent.w != 0 && ld_cg(&ws.state[ent.x]) == -1 && ld_cg(&ws.hlost[ent.z]) != r + 1;
     any_win |= won;
     if (won && ent.y == 0) ws.s[ent.x] = 2;

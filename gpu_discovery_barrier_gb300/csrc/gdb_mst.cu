@@ -84,7 +84,7 @@ __device__ __forceinline__ void zero_bytes(uint8_t* p, uint32_t n, const Warps& 
 //   and 16-byte zeroing of the marks; 2.02 with the rest, the pointer jumping
 //   four vertices per thread and the last round not run (mst_body).
 __device__ __forceinline__ void mst_lightest(const GraphView& G, const MstWs& ws, uint32_t round, int cur,
-                                             unsigned long long* my, unsigned long long& arcs) {
+                                             uint32_t nwarps, unsigned long long* my, unsigned long long& arcs) {
   const int lane = lane_id();
   auto offer = [&](uint32_t c, unsigned long long key) {
     if (key < ld_cg(&ws.best[c])) atomicMin(&ws.best[c], key);
@@ -159,11 +159,12 @@ __device__ __forceinline__ void mst_lightest(const GraphView& G, const MstWs& ws
       scan_group(v, mine ? ws.comp[v] : 0u, mine);
     }
   }
+  const uint32_t hk = chunk_width(G.nheavy_chunks, nwarps);
   for (;;) {
-    const uint32_t base = warp_grab(&ws.hcursor[cur]) * 32;
+    const uint32_t base = warp_grab(&ws.hcursor[cur]) * hk;
     if (base >= G.nheavy_chunks) break;
     const uint32_t ci = base + lane;
-    const bool have = ci < G.nheavy_chunks;
+    const bool have = (uint32_t)lane < hk && ci < G.nheavy_chunks;
     const uint4 ent = have ? __ldg(&G.heavy_chunk[ci]) : make_uint4(0, 0, 0, 0);
     uint32_t c = ent.x, rb = 0, re = 0;
     bool scan = have;
@@ -267,7 +268,7 @@ __device__ __forceinline__ void mst_body(Sync& s, const GraphView& G, const MstW
     {
       const int cur = t % 3, old = (t + 2) % 3;
       if (leader) ws.cursor[old] = ws.hcursor[old] = ws.hooks[old] = ws.alive[old] = 0;
-      mst_lightest(G, ws, round, cur, my, arcs);
+      mst_lightest(G, ws, round, cur, W.nwarps, my, arcs);
       if (!s.sync()) return;
       ++t;
     }
