@@ -126,7 +126,7 @@ __device__ __forceinline__ void mst_lightest(const GraphView& G, const MstWs& ws
     }
     __syncwarp();
   };
-  const uint32_t ngroups = (G.V + 31) / 32, grab = grab_of(ngroups);
+  const uint32_t ngroups = (G.V + 31) / 32, grab = sweep_grab(G, ngroups);
   for (;;) {
     const uint32_t g0 = warp_grab(&ws.cursor[cur]) * grab;
     if (g0 >= ngroups) break;
