@@ -397,9 +397,9 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
     // held the level up for hundreds of microseconds).  Accumulated as a
     // light vertex's count is: FP32 over a 32-arc step, then beyond floats --
     // a pair per step of the warp's successive chunks of one vertex, FP64
-    // over the warps in sacc, which the forward pass leaves idle -- and
-    // rounded once, by the warp that brings the vertex's last chunk, which
-    // also claims it.  (FP32 atomics of the chunks' sums lost what stays
+    // over the warps that share a vertex, in sacc, which the forward pass
+    // leaves idle -- and rounded once, by the warp that brings the vertex's
+    // last chunk, which also claims it.  (FP32 atomics of the chunks' sums lost what stays
     // under half a unit of a hub's count, and depended on their order.)
     const uint32_t hk = chunk_width(G.nheavy_chunks, W.nwarps);
     while (nhvbase < G.nheavy) {  // some left
@@ -443,17 +443,21 @@ __device__ __forceinline__ bool bc_forward(const GraphView& G, const Warps& W, c
         const uint32_t h = __shfl_sync(kFull, ent.z, o), nchunks = __shfl_sync(kFull, ent.w, o);
         bool claimed = false;
         if (lane == 0) {
-          if (part > 0.0) atomicAdd(&ws.sacc[u], part);
-          // as in heavy_done: the last one reads every warp's add
-          if (add_acq_rel(&ws.hpull[h], run) + run == nchunks) {
-            const double sum = __ldcg(&ws.sacc[u]);
-            ws.hpull[h] = 0;
-            claimed = sum > 0.0;
-            if (claimed) {
+          bool last = run == nchunks;  // all of them were this warp's
+          if (!last) {
+            if (part > 0.0) atomicAdd(&ws.sacc[u], part);
+            // as in heavy_done: the last one reads every warp's add
+            last = add_acq_rel(&ws.hpull[h], run) + run == nchunks;
+            if (last) {
+              part = __ldcg(&ws.sacc[u]);
               ws.sacc[u] = -0.0;
-              ws.st[u] = make_uint2((uint32_t)(Li + 1), __float_as_uint((float)sum));
-              next_arcs += degree(u);
+              ws.hpull[h] = 0;
             }
+          }
+          claimed = last && part > 0.0;
+          if (claimed) {
+            ws.st[u] = make_uint2((uint32_t)(Li + 1), __float_as_uint((float)part));
+            next_arcs += degree(u);
           }
         }
         if (__any_sync(kFull, claimed)) frontier_push_staged(G, out, qs, claimed, u);
